@@ -613,9 +613,10 @@ def cross_entropy(logits: Tensor, labels: Tensor, ignore_index: int) -> Tensor:
 
 def linear_cross_entropy(hidden: Tensor, weight: Tensor, bias: Optional[Tensor], labels: Tensor, ignore_index: int,
                          chunk_rows: int) -> Tensor:
-    from ..parallel.vocab_parallel import linear_cross_entropy as lce
+    from ..parallel.vocab_parallel import _epilogue_ce_ok, linear_cross_entropy as lce
+    # a vocabulary whose size is not a multiple of 8 only where the GEMM's epilogue can take it: there are no kernels for its logits
     fused = hidden.dtype in _16BIT and weight.dtype == hidden.dtype and hidden.size(-1) % 8 == 0 \
-        and weight.size(0) % 8 == 0
+        and (weight.size(0) % 8 == 0 or _epilogue_ce_ok(hidden, weight, bias, True, weight.size(0), 1))
     return lce(hidden, weight, bias, labels, ignore_index, chunk_rows, fused=fused)
 
 

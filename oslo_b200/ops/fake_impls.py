@@ -108,7 +108,9 @@ def register() -> None:
 
     @reg("oslo_b200::gemm_ce_grad")
     def _(a, b, b_mn, bias, labels, vocab_start, lse, scale):
-        return a.new_empty((a.size(0), b.size(1) if b_mn else b.size(0)))
+        n = b.size(1) if b_mn else b.size(0)
+        d = a.new_empty((a.size(0), (n + 7) // 8 * 8))       # rows at 16-byte boundaries
+        return d[:, :n] if n % 8 else d
 
     @reg("oslo_b200::error_word")
     def _(like):

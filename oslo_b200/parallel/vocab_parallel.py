@@ -65,17 +65,17 @@ def _epilogue_ce_ok(hidden: Tensor, weight: Tensor, bias: Optional[Tensor], fuse
     """The LM-head GEMM can do the cross-entropy work in its epilogue: kernels in use, 16-bit operands of one dtype,
     ``[vocab, hidden]`` weight with 16-byte aligned rows. The answer also selects the collective that combines the
     shards' statistics, so it must not depend on anything that differs between the ranks of the tensor-parallel group:
-    the row count is checked for ALL shards, not for this rank's."""
+    the row count is checked for ALL shards, not for this rank's. A whole vocabulary may have any size (GPT-2's and
+    GPT-Neo's 50257 words): the gradient matrix is then laid out with padded rows."""
     if not (fused and hidden.is_cuda and hidden.dtype in (torch.bfloat16, torch.float16)):
         return False
-    if not shard_rows_aligned(full_vocab, tp):
+    if tp > 1 and not shard_rows_aligned(full_vocab, tp):
         return False
     from ..config import get_config
     if not get_config().ce_in_gemm_epilogue:
         return False
     ok = (weight.dtype == hidden.dtype and weight.dim() == 2 and weight.stride(1) == 1 and weight.stride(0) % 8 == 0
-          and hidden.size(-1) % 8 == 0 and weight.data_ptr() % 16 == 0
-          and weight.size(0) % 8 == 0)      # rows of the [rows, vocab shard] gradient matrix stay 16-byte aligned
+          and hidden.size(-1) % 8 == 0 and weight.data_ptr() % 16 == 0)
     # (data_ptr alignment and strides of a shard come from the same allocator and the same slicing code on every rank)
     return ok and (bias is None or (bias.dtype == hidden.dtype and bias.is_contiguous()))
 
@@ -144,9 +144,10 @@ class _LinearCrossEntropy(torch.autograd.Function):
         n = hidden.size(0)
         scale = (g.float() / count) * valid.to(torch.float32)
         dx = torch.empty_like(hidden)
-        # the gradient GEMMs take [rows, vocab shard] operands: with a shard whose row count is not a multiple of 8 the
-        # rows of that matrix are not 16-byte aligned and the library products below are used instead (a local choice)
-        on_kernels = fused and hidden.is_cuda and weight.size(0) % 8 == 0
+        # the gradient GEMMs take [rows, vocab shard] operands whose rows start at 16-byte boundaries: those of
+        # gemm_ce_grad always do; logits of a shard whose row count is not a multiple of 8 do not, and the library
+        # products below are used instead (a local choice)
+        on_kernels = fused and hidden.is_cuda and (ctx.in_epilogue or weight.size(0) % 8 == 0)
         dw = None if on_kernels else torch.zeros_like(weight, dtype=torch.float32)
         dw_acc = None
         # weights whose gradient lives in the optimizer's flat buffer take the chunks' products there directly
@@ -182,7 +183,9 @@ class _LinearCrossEntropy(torch.autograd.Function):
                 else:                                                   # later chunks accumulate in the epilogue
                     cuda_ops.gemm(d, x, True, True, out=dw_acc, flags=cuda_ops.FLAG_OUT_FP32 | cuda_ops.FLAG_ACCUMULATE)
                 if db is not None:
-                    db += cuda_ops._ext().colsum(d)                     # fp32 column sums without an fp32 copy of d
+                    # fp32 column sums without an fp32 copy of d; with padded rows over the padding too, which is cut off
+                    whole = d if d.is_contiguous() else d.as_strided((d.size(0), d.stride(0)), d.stride())
+                    db += cuda_ops._ext().colsum(whole)[:d.size(1)]
             else:
                 dx[s:e] = (d @ weight).to(dx.dtype)
                 dw += d.float().t() @ x.float()

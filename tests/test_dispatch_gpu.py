@@ -1,0 +1,42 @@
+"""The rules that send a call to one kernel or another: sizes at the edges of each rule, against fp32 / fp64 PyTorch."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _ops():
+    from oslo_b200 import ops
+    from oslo_b200.ops import cuda_ops
+    return ops, cuda_ops
+
+
+def _rel(got, want):
+    return float((got.double() - want.double()).norm() / want.double().norm())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("vocab,rows,with_bias", [(5, 40, True), (33, 130, False), (1003, 300, True), (1007, 257, False), (50257, 200, False)])
+def test_loss_of_a_vocabulary_of_any_size(vocab, rows, with_bias, dtype):
+    """Vocabulary sizes that are no multiple of 8: loss and gradients on the GEMM kernels, whose gradient matrix has padded rows.
+    Each gradient is a sum of products of 16-bit factors rounded once more to 16 bits, so its 2-norm error is a few units of
+    2^-9 (bf16) or 2^-12 (fp16); four units allowed."""
+    ops, _ = _ops()
+    gen = torch.Generator(device="cuda").manual_seed(vocab)
+    mk = lambda *s, std: torch.randn(*s, device="cuda", generator=gen).mul_(std).to(dtype).requires_grad_(True)      # noqa: E731
+    h, w = mk(rows, 256, std=0.5), mk(vocab, 256, std=0.1)
+    b = mk(vocab, std=0.1) if with_bias else None
+    lab = torch.randint(0, vocab, (rows,), device="cuda", generator=gen)
+    lab[3], lab[4], lab[5] = -100, vocab - 1, 0
+    before = ops.load_ext().launch_count()
+    loss = ops.linear_cross_entropy(h, w, b, lab, chunk_rows=128)
+    assert ops.load_ext().launch_count() > before
+    (loss * 64).backward()
+    leaves = [t.detach().double().requires_grad_(True) for t in ((h, w, b) if with_bias else (h, w))]
+    logits = leaves[0] @ leaves[1].t() + (leaves[2] if with_bias else 0.0)
+    want = torch.nn.functional.cross_entropy(logits, lab, ignore_index=-100)
+    (want * 64).backward()
+    unit = 2.0 ** (-9 if dtype == torch.bfloat16 else -12)
+    assert abs(loss.item() - want.item()) < 16 * unit
+    for got, leaf in zip((h, w, b), leaves):
+        assert _rel(got.grad, leaf.grad) < 4 * unit, (vocab, got.shape, _rel(got.grad, leaf.grad))
