@@ -40,3 +40,27 @@ def test_loss_of_a_vocabulary_of_any_size(vocab, rows, with_bias, dtype):
     assert abs(loss.item() - want.item()) < 16 * unit
     for got, leaf in zip((h, w, b), leaves):
         assert _rel(got.grad, leaf.grad) < 4 * unit, (vocab, got.shape, _rel(got.grad, leaf.grad))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("cols", [8, 256, 264, 512, 520, 768, 1024, 1032, 2048, 2056, 4096, 4104, 6144, 6152, 8192])
+@pytest.mark.parametrize("rows", [1, 7, 1300])
+def test_layernorm_rows_at_the_edges_of_its_layouts(rows, cols, dtype):
+    """One size on each side of every (vectors per lane, warps per row) layout. Forward and input gradient are rounded once to the
+    storage type; the weight gradients sum `rows` products in fp32 before that."""
+    _, co = _ops()
+    if dtype == torch.float32 and cols > 4096:
+        pytest.skip("wider than the kernel takes in 32 bits")
+    gen = torch.Generator(device="cuda").manual_seed(rows * 10007 + cols)
+    mk = lambda *s: torch.randn(*s, device="cuda", generator=gen)                                               # noqa: E731
+    x, w, b, g = (mk(rows, cols) * 2 + 0.5).to(dtype), (1 + 0.1 * mk(cols)).to(dtype), mk(cols).to(dtype), mk(rows, cols).to(dtype)
+    leaves = [t.clone().requires_grad_(True) for t in (x, w, b)]
+    y = co.layer_norm(*leaves, 1e-5)
+    y.backward(g)
+    wide = [t.double().requires_grad_(True) for t in (x, w, b)]
+    want = torch.nn.functional.layer_norm(wide[0], (cols,), wide[1], wide[2], 1e-5)
+    want.backward(g.double())
+    unit = {torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -12, torch.float32: 2.0 ** -20}[dtype]
+    assert _rel(y, want) < 2 * unit
+    for leaf, ref in zip(leaves, wide):
+        assert _rel(leaf.grad, ref.grad) < 2 * unit, leaf.shape
