@@ -1,4 +1,4 @@
-// Flash-style attention (forward, backward) and single-query decode attention.
+// Flash-style attention (forward, backward).
 //
 // Scores never touch global memory: each CTA streams 64-wide blocks of the other operand through
 // shared memory (cp.async, padded rows so ldmatrix is bank-conflict free) and keeps its output
@@ -471,131 +471,6 @@ __global__ void __launch_bounds__(ATT_THREADS) flash_bwd_dkv_kernel(const AttnPa
   }
 }
 
-// ---------------------------------------------------------------------- decode attention (one query per row)
-// grid (splits, H, B); each CTA scans a slice of the cache with online softmax and writes a partial
-// (max, sum, out[D]) to the workspace; the combine kernel merges the slices.
-template <typename T>
-__global__ void __launch_bounds__(128) decode_attn_kernel(const T* __restrict__ q, const T* __restrict__ kc,
-                                                          const T* __restrict__ vc, const int* __restrict__ lengths,
-                                                          float* __restrict__ ws, int H, int Tmax, int D, int splits,
-                                                          float scale, int window, int* err) {
-  extern __shared__ float sm_dec[];
-  float* qs = sm_dec;             // [D]
-  float* red = qs + D;            // [4][D] per-warp partial outputs
-  float* stat = red + 4 * D;      // [4][2]
-  const int b = blockIdx.z, h = blockIdx.y, sp = blockIdx.x;
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  int len = lengths[b];
-  if (len < 0 || len > Tmax) {   // a length that does not fit the cache: never read past it
-    OSLO_REPORT_BOUNDS(err);
-    len = len < 0 ? 0 : Tmax;
-  }
-  int lo = 0;
-  if (window > 0) lo = max(0, len - window);
-  const int span = len - lo;
-  const int per = (span + splits - 1) / splits;
-  const int t0 = lo + sp * per, t1 = min(len, t0 + per);
-  const T* qp = q + (static_cast<long long>(b) * H + h) * D;
-  for (int d = threadIdx.x; d < D; d += 128) qs[d] = Mma<T>::to_f(qp[d]) * scale * LOG2E;
-  __syncthreads();
-  const T* kb = kc + (static_cast<long long>(b) * H + h) * Tmax * D;
-  const T* vb = vc + (static_cast<long long>(b) * H + h) * Tmax * D;
-  float m = -CUDART_INF_F, s = 0.f;
-  float acc[8];  // lane owns dims l*8.. (D <= 256) in 16-byte chunks
-#pragma unroll
-  for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-  const bool lane_active = l * 8 < D;
-  // each warp walks its keys in batches of KB: all K and V rows of a batch are requested before any of them is
-  // used, so a warp keeps 2 * KB 16-byte loads in flight instead of one (the scan is latency-bound otherwise)
-  constexpr int KB = 8;
-  for (int tb = t0 + w * KB; tb < t1; tb += 4 * KB) {
-    uint4 kraw[KB], vraw[KB];
-#pragma unroll
-    for (int j = 0; j < KB; ++j) {
-      const int t = tb + j;
-      if (lane_active && t < t1) {
-        kraw[j] = *reinterpret_cast<const uint4*>(kb + static_cast<long long>(t) * D + l * 8);
-        vraw[j] = *reinterpret_cast<const uint4*>(vb + static_cast<long long>(t) * D + l * 8);
-      } else {
-        kraw[j] = make_uint4(0, 0, 0, 0);
-        vraw[j] = make_uint4(0, 0, 0, 0);
-      }
-    }
-    float dot[KB];
-#pragma unroll
-    for (int j = 0; j < KB; ++j) {
-      const T* e = reinterpret_cast<const T*>(&kraw[j]);
-      float d = 0.f;
-      if (lane_active) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) d += Mma<T>::to_f(e[i]) * qs[l * 8 + i];
-      }
-      dot[j] = d;
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-#pragma unroll
-      for (int j = 0; j < KB; ++j) dot[j] += __shfl_xor_sync(0xffffffffu, dot[j], off);
-    }
-    float mn = m;
-#pragma unroll
-    for (int j = 0; j < KB; ++j) {
-      if (tb + j >= t1) dot[j] = -CUDART_INF_F;
-      mn = fmaxf(mn, dot[j]);
-    }
-    const float a = exp2f(m - mn);   // m = -inf on the first batch: a = 0 and s, acc are 0 anyway
-    float ps = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] *= a;
-#pragma unroll
-    for (int j = 0; j < KB; ++j) {
-      const float pr = exp2f(dot[j] - mn);
-      ps += pr;
-      const T* e = reinterpret_cast<const T*>(&vraw[j]);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) acc[i] += pr * Mma<T>::to_f(e[i]);
-    }
-    s = s * a + ps;
-    m = mn;
-  }
-  if (l == 0) { stat[w * 2] = m; stat[w * 2 + 1] = s; }
-  __syncthreads();
-  float gm = fmaxf(fmaxf(stat[0], stat[2]), fmaxf(stat[4], stat[6]));
-  const float mine = (m == -CUDART_INF_F) ? 0.f : exp2f(m - gm);
-  if (lane_active) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) red[w * D + l * 8 + i] = acc[i] * mine;
-  }
-  __syncthreads();
-  float gs = 0.f;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) gs += (stat[i * 2] == -CUDART_INF_F) ? 0.f : stat[i * 2 + 1] * exp2f(stat[i * 2] - gm);
-  float* out = ws + ((static_cast<long long>(b) * H + h) * splits + sp) * (D + 2);
-  for (int d = threadIdx.x; d < D; d += 128) out[d] = red[d] + red[D + d] + red[2 * D + d] + red[3 * D + d];
-  if (threadIdx.x == 0) { out[D] = gm; out[D + 1] = gs; }
-}
-template <typename T>
-__global__ void decode_combine_kernel(const float* __restrict__ ws, T* __restrict__ o, int D, int splits) {
-  const long long bh = blockIdx.x;
-  const float* base = ws + bh * splits * (D + 2);
-  float gm = -CUDART_INF_F;
-  for (int s = 0; s < splits; ++s) gm = fmaxf(gm, base[s * (D + 2) + D]);
-  float tot = 0.f;
-  for (int s = 0; s < splits; ++s) {
-    const float m = base[s * (D + 2) + D];
-    if (m != -CUDART_INF_F) tot += base[s * (D + 2) + D + 1] * exp2f(m - gm);
-  }
-  const float inv = tot > 0.f ? 1.f / tot : 0.f;
-  for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    float a = 0.f;
-    for (int s = 0; s < splits; ++s) {
-      const float m = base[s * (D + 2) + D];
-      if (m != -CUDART_INF_F) a += base[s * (D + 2) + d] * exp2f(m - gm);
-    }
-    o[bh * D + d] = Mma<T>::from_f(a * inv);
-  }
-}
-
 template <typename K>
 static int set_smem(K kernel, size_t bytes) {
   return static_cast<int>(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
@@ -696,26 +571,4 @@ extern "C" int oslo_flash_bwd(const void* q, const void* k, const void* v, const
   p.o = o; p.dout = dout; p.lse = const_cast<float*>(lse); p.delta = delta;
   p.dq = dq; p.dk = dk; p.dv = dv; p.do_sb = do_sb; p.do_sh = do_sh; p.do_ss = do_ss;
   ATT_DISPATCH(dtype, D, { return launch_bwd<T, HD>(p, delta, st); })
-}
-
-extern "C" int oslo_decode_attn(const void* q, const void* kc, const void* vc, void* o, const int* lengths, float* ws,
-                                int B, int H, int T, int D, int splits, float scale, int window, int dtype,
-                                int* err_word, cudaStream_t st) {
-  if (B * H == 0) return 0;
-  if (D % 8 || D > 256) return -3;
-  const size_t smem = (D + 4 * D + 8) * sizeof(float);
-  dim3 grid(splits, H, B);
-  if (dtype == OSLO_DT_BF16) {
-    decode_attn_kernel<__nv_bfloat16><<<grid, 128, smem, st>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)kc,
-                                                               (const __nv_bfloat16*)vc, lengths, ws, H, T, D, splits,
-                                                               scale, window, err_word);
-    decode_combine_kernel<__nv_bfloat16><<<B * H, 128, 0, st>>>(ws, (__nv_bfloat16*)o, D, splits);
-  } else if (dtype == OSLO_DT_FP16) {
-    decode_attn_kernel<__half><<<grid, 128, smem, st>>>((const __half*)q, (const __half*)kc, (const __half*)vc, lengths,
-                                                        ws, H, T, D, splits, scale, window, err_word);
-    decode_combine_kernel<__half><<<B * H, 128, 0, st>>>(ws, (__half*)o, D, splits);
-  } else {
-    return -2;
-  }
-  return static_cast<int>(cudaGetLastError());
 }

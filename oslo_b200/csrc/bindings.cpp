@@ -203,38 +203,62 @@ Tensor gemm_ce_grad(const Tensor& a, const Tensor& b, int64_t b_mn, const option
   return d;
 }
 
-// y = act(a @ b^T + bias) for few rows (decode steps): split-K GEMM into fp32 planes, then one finalisation
-// kernel that sums them in a fixed order. Falls back to the ordinary GEMM when splitting the k range gains nothing.
-// `gelu_from`: -1 = no activation, c >= 0 = tanh-GeLU on output columns >= c (0 = all of them), which lets one GEMM
-// serve several layers that share an input when only the last of them is followed by the activation.
+// y [M, N] = act([x1 | x2] @ w^T + bias) + res for M <= 64 rows (decode steps); w [N, K1 + K2], or [K1 + K2, N] with `w_kn`, or up to
+// three equally large matrices one below the other. `gelu_from`: -1 = no activation, c >= 0 = tanh-GeLU on output columns >= c (0 = all
+// of them), which lets one product serve several layers that share an input when only the last of them is followed by the activation.
+// `ln_w` (M <= 8, M * K1 <= 8192): LayerNorm(x1) is what is multiplied.
+Tensor few_rows(const Tensor& x1, const optional<Tensor>& x2, const std::vector<Tensor>& w, int64_t w_kn, const optional<Tensor>& bias,
+                int64_t gelu_from, const optional<Tensor>& res, const optional<Tensor>& ln_w, const optional<Tensor>& ln_b, double eps) {
+  check_2d_operand(x1, "x1");
+  TORCH_CHECK(!w.empty() && w.size() <= 3, "few_rows: one to three weights");
+  const bool two = x2.has_value() && x2->defined();
+  if (two) check_2d_operand(*x2, "x2");
+  const int64_t M = x1.size(0), K1 = x1.size(1), K2 = two ? x2->size(1) : 0, parts = static_cast<int64_t>(w.size());
+  const int64_t N = (w_kn ? w[0].size(1) : w[0].size(0)) * parts;
+  for (const Tensor& part : w) {
+    check_2d_operand(part, "w");
+    TORCH_CHECK(part.sizes() == w[0].sizes() && part.stride(0) == w[0].stride(0) && part.scalar_type() == x1.scalar_type() &&
+                    (w_kn ? part.size(0) : part.size(1)) == K1 + K2 && part.device() == x1.device(), "few_rows: shapes or dtypes do not match");
+  }
+  TORCH_CHECK(!two || (x2->size(0) == M && x2->scalar_type() == x1.scalar_type() && x2->device() == x1.device()), "few_rows: x2 does not match x1");
+  TORCH_CHECK(x1.scalar_type() == at::kBFloat16 || x1.scalar_type() == at::kHalf, "few_rows inputs must be bf16 or fp16");
+  const auto vec = [&](const optional<Tensor>& t, int64_t n, const char* what) -> const void* {
+    if (!t.has_value() || !t->defined()) return nullptr;
+    TORCH_CHECK(t->numel() == n && t->scalar_type() == x1.scalar_type() && t->is_contiguous() && t->device() == x1.device(), "bad ", what);
+    return t->data_ptr();
+  };
+  const void* b = vec(bias, N, "bias");
+  const void* lw = vec(ln_w, K1, "LayerNorm weight");
+  const void* lb = vec(ln_b, K1, "LayerNorm bias");
+  TORCH_CHECK(lw || !lb, "few_rows: a LayerNorm bias needs its weight");
+  const bool has_res = res.has_value() && res->defined();
+  if (has_res)
+    TORCH_CHECK(res->dim() == 2 && res->size(0) == M && res->size(1) == N && res->stride(1) == 1 &&
+                    res->scalar_type() == x1.scalar_type() && res->device() == x1.device(), "bad residual");
+  c10::cuda::CUDAGuard guard(x1.device());
+  if (M > 8 && two && K1 % 64)                 // a k block of the tensor-core kernel comes from one of the inputs
+    return few_rows(at::cat({x1, *x2}, 1), optional<Tensor>(), w, w_kn, bias, gelu_from, res, ln_w, ln_b, eps);
+  if (M > 8 && parts > 1 && (N / parts) % 128) // ... and a tile from one of the weights
+    return few_rows(x1, x2, {at::cat(w, 0)}, w_kn, bias, gelu_from, res, ln_w, ln_b, eps);
+  Tensor y = at::empty({M, N}, x1.options());
+  auto& st = dev_state(x1.get_device());
+  check_rc(oslo_few_rows(x1.data_ptr(), static_cast<int>(x1.stride(0)), static_cast<int>(K1), two ? x2->data_ptr() : nullptr,
+                         two ? static_cast<int>(x2->stride(0)) : 0, static_cast<int>(K2), w[0].data_ptr(),
+                         parts > 1 ? w[1].data_ptr() : nullptr, parts > 2 ? w[2].data_ptr() : nullptr, static_cast<int>(parts),
+                         static_cast<int>(w[0].stride(0)), static_cast<int>(w_kn), b, has_res ? res->data_ptr() : nullptr,
+                         has_res ? static_cast<int>(res->stride(0)) : 0, lw, lb, static_cast<float>(eps), y.data_ptr(),
+                         static_cast<int>(N), static_cast<int>(M), static_cast<int>(N), static_cast<int>(gelu_from), dt_code(x1),
+                         st.err.data_ptr<int>(), usable_sms(st), cur_stream()), "few_rows");
+  return y;
+}
 Tensor gemm_small_m(const Tensor& a, const Tensor& b, int64_t b_mn, const optional<Tensor>& bias, int64_t gelu_from) {
-  check_2d_operand(a, "a");
-  check_2d_operand(b, "b");
-  TORCH_CHECK(a.scalar_type() == b.scalar_type(), "a and b must share a dtype");
-  TORCH_CHECK(a.scalar_type() == at::kBFloat16 || a.scalar_type() == at::kHalf, "gemm inputs must be bf16 or fp16");
-  c10::cuda::CUDAGuard guard(a.device());
-  const int64_t M = a.size(0), K = a.size(1);
-  const int64_t N = b_mn ? b.size(1) : b.size(0), Kb = b_mn ? b.size(0) : b.size(1);
-  TORCH_CHECK(K == Kb, "contraction sizes differ: ", K, " vs ", Kb);
-  auto& st = dev_state(a.get_device());
-  const int split = std::max(1, oslo_gemm_split_k_for(static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), usable_sms(st)));
-  const bool has_bias = bias.has_value() && bias->defined();
-  if (has_bias)
-    TORCH_CHECK(bias->numel() == N && bias->scalar_type() == a.scalar_type() && bias->is_contiguous(), "bad bias");
-  if (split <= 1 && gelu_from <= 0) {
+  if (a.size(0) > 64 || (b_mn && b.size(1) % 8)) {
+    TORCH_CHECK(gelu_from <= 0, "gemm_small_m: an activation on some columns needs at most 64 rows");
+    const bool has_bias = bias.has_value() && bias->defined();
     const int64_t fl = (has_bias ? GEMM_FLAG_BIAS : 0) | (gelu_from == 0 ? GEMM_FLAG_GELU : 0) | (gelu_from == OSLO_ACT_RELU2 ? GEMM_FLAG_RELU2 : 0);
     return gemm(a, b, 0, b_mn, bias, optional<Tensor>(), optional<Tensor>(), optional<Tensor>(), fl, 1.0);
   }
-  Tensor ws = at::empty({split, M, N}, a.options().dtype(at::kFloat));
-  check_rc(oslo_gemm_splitk_16bit(a.data_ptr(), b.data_ptr(), ws.data_ptr<float>(), static_cast<int>(M),
-                                  static_cast<int>(N), static_cast<int>(K), static_cast<int>(a.stride(0)),
-                                  static_cast<int>(b.stride(0)), static_cast<int>(N), 0, static_cast<int>(b_mn),
-                                  a.scalar_type() == at::kHalf ? 1 : 0, split, st.err.data_ptr<int>(), usable_sms(st),
-                                  cur_stream()), "gemm_splitk");
-  Tensor y = at::empty({M, N}, a.options());
-  check_rc(oslo_splitk_finalize(ws.data_ptr<float>(), has_bias ? bias->data_ptr() : nullptr, y.data_ptr(), M,
-                                static_cast<int>(N), split, static_cast<int>(gelu_from), dt_code(a), cur_stream()), "splitk_finalize");
-  return y;
+  return few_rows(a, optional<Tensor>(), {b}, b_mn, bias, gelu_from, optional<Tensor>(), optional<Tensor>(), optional<Tensor>(), 0.0);
 }
 
 std::tuple<Tensor, Tensor, Tensor> layernorm_fwd(const Tensor& x, const Tensor& w, const optional<Tensor>& b, double eps) {
@@ -503,23 +527,41 @@ std::tuple<Tensor, Tensor, Tensor> flash_bwd(const Tensor& dout, const Tensor& q
   return {dq, dk, dv};
 }
 
-Tensor decode_attn(const Tensor& q, const Tensor& kc, const Tensor& vc, const Tensor& lengths, double scale,
-                   int64_t window) {
-  TORCH_CHECK(q.is_cuda() && q.dim() == 3 && q.is_contiguous(), "decode_attn: q must be contiguous [B,H,D]");
-  TORCH_CHECK(kc.dim() == 4 && kc.is_contiguous() && vc.is_contiguous(), "decode_attn: caches must be contiguous [B,H,T,D]");
-  TORCH_CHECK(lengths.scalar_type() == at::kInt && lengths.is_contiguous() && lengths.numel() == q.size(0), "bad lengths");
+// q (and the new token's k, v) [B, H, D] with contiguous D; caches [B, H, T, D]. With k and v: rotary on q and k (rotary_dim > 0, at
+// positions[b]) and the append at write_index[0] happen in the same kernel.
+Tensor decode_step_attn(const Tensor& q, const optional<Tensor>& k, const optional<Tensor>& v, Tensor kc, Tensor vc, const Tensor& lengths,
+                        const optional<Tensor>& positions, const optional<Tensor>& write_index, int64_t rotary_dim, double base,
+                        double scale, int64_t window) {
+  TORCH_CHECK(q.is_cuda() && q.dim() == 3 && q.stride(2) == 1, "decode_attn: q must be [B,H,D] with contiguous D");
+  TORCH_CHECK(kc.dim() == 4 && kc.is_contiguous() && vc.is_contiguous() && kc.sizes() == vc.sizes(), "decode_attn: caches must be contiguous [B,H,T,D]");
+  TORCH_CHECK(kc.size(0) == q.size(0) && kc.size(1) == q.size(1) && kc.size(3) == q.size(2) && kc.scalar_type() == q.scalar_type() &&
+                  vc.scalar_type() == q.scalar_type() && kc.device() == q.device() && vc.device() == q.device(), "decode_attn: q and caches do not match");
+  TORCH_CHECK(lengths.scalar_type() == at::kInt && lengths.is_contiguous() && lengths.numel() == q.size(0) && lengths.is_cuda(), "bad lengths");
+  const bool append = k.has_value() && k->defined();
+  if (append) {
+    TORCH_CHECK(v.has_value() && v->defined() && k->sizes() == q.sizes() && v->sizes() == q.sizes() && k->stride(2) == 1 && v->stride(2) == 1 &&
+                    k->scalar_type() == q.scalar_type() && v->scalar_type() == q.scalar_type() && k->device() == q.device() &&
+                    v->device() == q.device(), "decode_attn: k and v must be like q");
+    TORCH_CHECK(write_index.has_value() && write_index->scalar_type() == at::kLong && write_index->numel() >= 1 && write_index->is_cuda(), "bad write index");
+    TORCH_CHECK(rotary_dim == 0 || (positions.has_value() && positions->scalar_type() == at::kInt && positions->is_contiguous() &&
+                                    positions->numel() == q.size(0) && positions->is_cuda()), "bad rotary positions");
+  }
   c10::cuda::CUDAGuard guard(q.device());
-  const int B = q.size(0), H = q.size(1), D = q.size(2), T = kc.size(2);
-  const int sms = dev_state(q.get_device()).sms;
-  int splits = std::max(1, std::min(32, (2 * sms) / std::max(1, B * H)));
-  splits = std::min(splits, std::max(1, T / 32));   // at least one 8-key batch per warp and slice
-  Tensor ws = at::empty({B, H, splits, D + 2}, q.options().dtype(at::kFloat));
-  Tensor o = at::empty_like(q);
-  check_rc(oslo_decode_attn(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), o.data_ptr(), lengths.data_ptr<int>(),
-                            ws.data_ptr<float>(), B, H, T, D, splits, static_cast<float>(scale),
-                            static_cast<int>(window), dt_code(q), dev_state(q.get_device()).err.data_ptr<int>(),
-                            cur_stream(2)), "decode_attn");
+  Tensor o = at::empty(q.sizes(), q.options());
+  auto& st = dev_state(q.get_device());
+  check_rc(oslo_decode_attn(q.data_ptr(), append ? k->data_ptr() : nullptr, append ? v->data_ptr() : nullptr, kc.data_ptr(), vc.data_ptr(),
+                            o.data_ptr(), q.stride(0), q.stride(1), append ? k->stride(0) : 0, append ? k->stride(1) : 0,
+                            append ? v->stride(0) : 0, append ? v->stride(1) : 0, lengths.data_ptr<int>(),
+                            append && rotary_dim ? positions->data_ptr<int>() : nullptr,
+                            append ? reinterpret_cast<const long long*>(write_index->data_ptr<int64_t>()) : nullptr,
+                            static_cast<int>(q.size(0)), static_cast<int>(q.size(1)), static_cast<int>(kc.size(2)),
+                            static_cast<int>(q.size(2)), static_cast<int>(rotary_dim), static_cast<float>(base), static_cast<float>(scale),
+                            static_cast<int>(window), dt_code(q), st.sms, st.err.data_ptr<int>(), cur_stream()), "decode_attn");
   return o;
+}
+Tensor decode_attn(const Tensor& q, const Tensor& kc, const Tensor& vc, const Tensor& lengths, double scale, int64_t window) {
+  TORCH_CHECK(q.is_contiguous(), "decode_attn: q must be contiguous [B,H,D]");
+  return decode_step_attn(q, optional<Tensor>(), optional<Tensor>(), kc, vc, lengths, optional<Tensor>(), optional<Tensor>(), 0, 1.0, scale, window);
 }
 
 // GEMM fused with a collective over the symmetric buffer of a tensor-parallel group (fused_comm_gemm.cu).
@@ -627,32 +669,11 @@ void dp_all_gather(const Tensor& like, int64_t peer_ptrs_dev, int64_t mc_ptr, in
            "dp_all_gather");
 }
 
-// y [M, N] = act([x1 | x2] @ w^T + bias) for M <= 4 rows; w [N, K1 + K2]; x1 / x2 are 2-D with contiguous last dims
+// y [M, N] = act([x1 | x2] @ w^T + bias) (+ res) for M <= 4 rows; w [N, K1 + K2]; x1 / x2 are 2-D with contiguous last dims
 Tensor gemv_rows(const Tensor& x1, const optional<Tensor>& x2, const Tensor& w, const optional<Tensor>& bias,
                  int64_t gelu_from, const optional<Tensor>& res) {
-  check_2d_operand(x1, "x1");
-  check_2d_operand(w, "w");
-  const bool two = x2.has_value() && x2->defined();
-  if (two) check_2d_operand(*x2, "x2");
-  const int64_t M = x1.size(0), K1 = x1.size(1), K2 = two ? x2->size(1) : 0, N = w.size(0);
-  TORCH_CHECK(w.size(1) == K1 + K2 && (!two || x2->size(0) == M), "gemv_rows: shapes do not match");
-  TORCH_CHECK(x1.scalar_type() == w.scalar_type() && (!two || x2->scalar_type() == w.scalar_type()), "gemv_rows: dtypes differ");
-  const bool has_bias = bias.has_value() && bias->defined();
-  if (has_bias) TORCH_CHECK(bias->numel() == N && bias->scalar_type() == w.scalar_type() && bias->is_contiguous(), "bad bias");
-  const bool has_res = res.has_value() && res->defined();
-  if (has_res)
-    TORCH_CHECK(res->dim() == 2 && res->size(0) == M && res->size(1) == N && res->stride(1) == 1 &&
-                    res->scalar_type() == w.scalar_type(), "bad residual");
-  c10::cuda::CUDAGuard guard(x1.device());
-  Tensor y = at::empty({M, N}, x1.options());
-  auto& st = dev_state(x1.get_device());
-  check_rc(oslo_gemv_rows(x1.data_ptr(), static_cast<int>(x1.stride(0)), static_cast<int>(K1),
-                          two ? x2->data_ptr() : nullptr, two ? static_cast<int>(x2->stride(0)) : 0, static_cast<int>(K2),
-                          w.data_ptr(), static_cast<int>(w.stride(0)), has_bias ? bias->data_ptr() : nullptr,
-                          has_res ? res->data_ptr() : nullptr, has_res ? static_cast<int>(res->stride(0)) : 0, y.data_ptr(),
-                          static_cast<int>(N), static_cast<int>(M), static_cast<int>(N), static_cast<int>(gelu_from),
-                          dt_code(x1), usable_sms(st), cur_stream()), "gemv_rows");
-  return y;
+  TORCH_CHECK(x1.dim() == 2 && x1.size(0) <= 4 && w.dim() == 2 && w.size(0) % 4 == 0, "gemv_rows: at most 4 rows, a multiple of 4 columns");
+  return few_rows(x1, x2, {w}, 0, bias, gelu_from, res, optional<Tensor>(), optional<Tensor>(), 0.0);
 }
 
 // GPT-J rotary on q, k ([B, H*D] row slices) + append of k, v to the static cache at the device-side position
@@ -963,7 +984,7 @@ Tensor gemv_stacked(const Tensor& x, const Tensor& w) {
                   x.size(2) == w.size(2) && x.scalar_type() == w.scalar_type(), "gemv_stacked: operands");
   c10::cuda::CUDAGuard guard(x.device());
   Tensor out = at::empty({x.size(0), x.size(1), w.size(1)}, x.options());
-  check_rc(oslo_gemv_stacked(x.data_ptr(), static_cast<int>(x.stride(1)), x.stride(0), w.data_ptr(), static_cast<int>(w.size(2)),
+  check_rc(oslo_few_rows_stacked(x.data_ptr(), static_cast<int>(x.stride(1)), x.stride(0), w.data_ptr(), static_cast<int>(w.size(2)),
                              w.size(1) * w.size(2), out.data_ptr(), static_cast<int>(x.size(0)), static_cast<int>(x.size(1)),
                              static_cast<int>(w.size(1)), static_cast<int>(w.size(2)), dt_code(x), dev_state(x.get_device()).sms,
                              cur_stream()), "gemv_stacked");
@@ -1770,6 +1791,10 @@ TORCH_LIBRARY(oslo_b200, m) {
   m.def("flash_bwd(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse, float scale, bool causal, int window, Tensor? kpm, int impl=1) -> (Tensor, Tensor, Tensor)");
   m.def("decode_attn(Tensor q, Tensor kc, Tensor vc, Tensor lengths, float scale, int window) -> Tensor");
   m.def("gemm_comm(Tensor a, Tensor b, int a_mn, int b_mn, Tensor? bias, Tensor? aux, Tensor(a!)? aux_out, Tensor(b!)? out, int flags, float alpha, int M, int N, int K, int peer_bufs_dev, int own_buf, int mc_base, int data_off, int flag_off, int flag_bytes, int rank, int world, int epoch, int done_base, int mode, bool use_multimem, Tensor(c!)? trace) -> int");
+  m.def("few_rows(Tensor x1, Tensor? x2, Tensor[] w, int w_kn, Tensor? bias, int gelu_from, Tensor? res=None, Tensor? ln_w=None, "
+        "Tensor? ln_b=None, float eps=0.0) -> Tensor");
+  m.def("decode_step_attn(Tensor q, Tensor? k, Tensor? v, Tensor(a!) kc, Tensor(b!) vc, Tensor lengths, Tensor? positions, "
+        "Tensor? write_index, int rotary_dim, float base, float scale, int window) -> Tensor");
   m.def("gemv_rows(Tensor x1, Tensor? x2, Tensor w, Tensor? bias, int gelu_from, Tensor? res=None) -> Tensor");
   m.def("rotary_append(Tensor q, Tensor k, Tensor v, Tensor(a!) kc, Tensor(b!) vc, Tensor lengths, Tensor write_index, int rotary_dim, float base) -> Tensor");
   m.def("vocab_embed(Tensor ids, Tensor weight, int lo, int hi, int peer_ptrs_dev, int mc_ptr, int signal_ptrs_dev, Tensor(a!) counters, int half_bytes, int rank, int world, bool use_multimem) -> Tensor");
@@ -1844,6 +1869,8 @@ TORCH_LIBRARY_IMPL(oslo_b200, CUDA, m) {
   m.impl("flash_bwd", &flash_bwd);
   m.impl("decode_attn", &decode_attn);
   m.impl("gemm_comm", &gemm_comm);
+  m.impl("few_rows", &few_rows);
+  m.impl("decode_step_attn", &decode_step_attn);
   m.impl("gemv_rows", &gemv_rows);
   m.impl("rotary_append", &rotary_append);
   m.impl("vocab_embed", &vocab_embed);

@@ -1,13 +1,9 @@
-// Kernels of the single-token decode step (a handful of rows per call). Everything here is bound by how fast
-// weights and the KV cache stream out of HBM and by launch count, not by math, so the kernels are plain
-// wide-load CUDA-core code with as many 16-byte loads in flight as the register file allows, and they fuse what
-// the eager path runs as separate launches:
-//   * gemv_rows_kernel: y[m, n] = act(sum_k [x1 | x2][m, k] * W[n, k] + bias[n]) + res[m, n] for m <= 4 (beyond that the CUDA
-//     cores cannot keep up with HBM and the tensor-core split-k path takes over). One block owns four output
-//     columns and the whole k range, so there is no second pass; the input may come in two pieces
-//     (attention output and MLP activation feeding the merged out_proj / fc_out product of a parallel block).
+// Kernels of the single-token decode step: bound by how fast the KV cache streams out of HBM and by launch count, not by math. The
+// weight products are in few_rows_sm100.cu.
 //   * rotary_append_kernel: GPT-J rotary on q and k of the new token, q to a contiguous buffer, k and v written
 //     into the static cache at the position held in device memory.
+//   * decode_attn_kernel: attention of one query per row over the cache, with the rotary and the append of the new token inside
+//     when it is given one.
 //
 // Reference behaviour covered: one iteration of the token loop of oslo/generation_utils.py:1269-1361 through a
 // GPT-J block (oslo/models/gptj/modeling_gptj.py:196-320: rotary at the cache offset, torch.cat cache growth,
@@ -32,116 +28,6 @@ template <> struct DCvt<__half> {
   static __device__ __forceinline__ __half from(float v) { return __float2half_rn(v); }
   static __device__ __forceinline__ float to(__half v) { return __half2float(v); }
 };
-
-__device__ __forceinline__ uint4 ld_stream_16(const void* p) {   // weights are read once: keep them out of L1
-  uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ float gelu_tanh_dec(float x) {
-  const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
-  float t;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(u));
-  return 0.5f * x * (1.0f + t);
-}
-
-constexpr int GV_COLS = 4;      // output columns per warp
-constexpr int GV_THREADS = 256;
-
-// accumulate the k range [k_begin, K) in steps of k_step for GV_COLS weight rows; two chunks per iteration so that
-// each lane keeps 2 * GV_COLS 16-byte weight loads in flight
-template <typename T, int MR>
-__device__ __forceinline__ void gemv_segment(const T* __restrict__ x, int ldx, int K, const T* __restrict__ w, int ldw,
-                                             int m_valid, int k_begin, int k_step, float (&acc)[GV_COLS][MR]) {
-  for (int k = k_begin; k < K; k += 2 * k_step) {
-    const int kb = k + k_step;
-    const bool second = kb < K;
-    uint4 wv[2][GV_COLS];
-#pragma unroll
-    for (int c = 0; c < GV_COLS; ++c) {
-      wv[0][c] = ld_stream_16(w + static_cast<size_t>(c) * ldw + k);
-      wv[1][c] = second ? ld_stream_16(w + static_cast<size_t>(c) * ldw + kb) : make_uint4(0, 0, 0, 0);
-    }
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      if (u == 1 && !second) break;
-      const int kk = u ? kb : k;
-#pragma unroll
-      for (int m = 0; m < MR; ++m) {
-        if (m < m_valid) {
-          const uint4 xv = *reinterpret_cast<const uint4*>(x + static_cast<size_t>(m) * ldx + kk);
-          const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w};
-#pragma unroll
-          for (int c = 0; c < GV_COLS; ++c) {
-            const uint32_t ww[4] = {wv[u][c].x, wv[u][c].y, wv[u][c].z, wv[u][c].w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const float2 a = DCvt<T>::to2(xw[j]);
-              const float2 b = DCvt<T>::to2(ww[j]);
-              acc[c][m] = fmaf(a.x, b.x, acc[c][m]);
-              acc[c][m] = fmaf(a.y, b.y, acc[c][m]);
-            }
-          }
-        }
-      }
-    }
-  }
-}
-
-// W is [N, K1 + K2] with row stride ldw (K-major); x1 [m, K1], x2 [m, K2] (x2 may be null); N % 4 == 0, K % 8 == 0.
-// One block per group of GV_COLS output columns: its 8 warps interleave over the k range (each lane 8 elements of
-// every 2048-element stripe), so consecutive warps read consecutive 512-byte pieces of the same weight rows.
-template <typename T, int MR>
-__global__ void __launch_bounds__(GV_THREADS) gemv_rows_kernel(const T* __restrict__ x1, int ld1, int K1,
-                                                               const T* __restrict__ x2, int ld2, int K2,
-                                                               const T* __restrict__ W, int ldw,
-                                                               const T* __restrict__ bias,
-                                                               const T* __restrict__ res, int ldr, T* __restrict__ out,
-                                                               int ldo, int N, int m_valid, int gelu_from,
-                                                               long long sx, long long sw, long long so) {
-  x1 += blockIdx.y * sx;                        // stacked products: one per blockIdx.y
-  W += blockIdx.y * sw;
-  out += blockIdx.y * so;
-  __shared__ float red[GV_THREADS / 32][GV_COLS * MR];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int k_begin = threadIdx.x * 8, k_step = GV_THREADS * 8;
-  for (int n0 = blockIdx.x * GV_COLS; n0 < N; n0 += gridDim.x * GV_COLS) {
-    float acc[GV_COLS][MR];
-#pragma unroll
-    for (int c = 0; c < GV_COLS; ++c)
-#pragma unroll
-      for (int m = 0; m < MR; ++m) acc[c][m] = 0.f;
-    const T* w = W + static_cast<size_t>(n0) * ldw;
-    gemv_segment<T, MR>(x1, ld1, K1, w, ldw, m_valid, k_begin, k_step, acc);
-    if (x2 != nullptr) gemv_segment<T, MR>(x2, ld2, K2, w + K1, ldw, m_valid, k_begin, k_step, acc);
-#pragma unroll
-    for (int c = 0; c < GV_COLS; ++c)
-#pragma unroll
-      for (int m = 0; m < MR; ++m) {
-        float v = acc[c][m];
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-        if (lane == 0) red[warp][c * MR + m] = v;
-      }
-    __syncthreads();
-    if (threadIdx.x < GV_COLS * MR) {
-      const int c = threadIdx.x / MR, m = threadIdx.x % MR;
-      float v = 0.f;
-#pragma unroll
-      for (int wv = 0; wv < GV_THREADS / 32; ++wv) v += red[wv][threadIdx.x];
-      if (m < m_valid) {
-        const int n = n0 + c;
-        if (bias) v += DCvt<T>::to(bias[n]);
-        if (gelu_from >= 0 && n >= gelu_from) v = gelu_tanh_dec(v);
-        if (gelu_from == OSLO_ACT_RELU2) { v = fmaxf(v, 0.f); v *= v; }
-        if (res) v += DCvt<T>::to(res[static_cast<size_t>(m) * ldr + n]);
-        out[static_cast<size_t>(m) * ldo + n] = DCvt<T>::from(v);
-      }
-    }
-    __syncthreads();
-  }
-}
 
 // One block per (batch row, head): rotary (pairs (2i, 2i+1) of the first rotary_dim dims, position pos[b]) on q and
 // k; q -> q_out [B, H, D]; k, v -> cache[b, h, write_index[0], :]. q/k/v rows are [H * D] slices with row strides.
@@ -183,55 +69,291 @@ __global__ void rotary_append_kernel(const T* __restrict__ q, const T* __restric
   }
 }
 
+// Attention of one query per (row, head) over the cache. The splits of a row's keys are the CTAs of a cluster: they merge their
+// (max, sum, output) through distributed shared memory, so there is no workspace and no second kernel.
+// LPK lanes read a key (eight dims each) and a warp 32 / LPK keys at once, so a narrow head leaves no lane idle. Every lane fetches its
+// own pieces of K and V with cp.async, DA_STAGES - 1 batches of DA_KEYS keys ahead: shared memory is a private queue, without barriers,
+// and keeps up to 128 KB per SM on their way. With `k` given, the new token's key and value are rotated (the first rotary_dim
+// dims), written to the cache at write_index[0] by the first split, and taken from registers by whichever split reaches that position.
+struct DecodeAttn {
+  const void* q; const void* k; const void* v;          // [B, H, D] by strides (b, h); k, v may be null
+  void* kc; void* vc; void* o;                          // caches [B, H, T, D], result [B, H, D]
+  const int* lengths; const int* positions;             // keys per row, the new token's among them; its rotary position
+  const long long* write_index;
+  int* err;
+  long long q_sb, q_sh, k_sb, k_sh, v_sb, v_sh;
+  float scale, log2_base;
+  int H, T, D, splits, window, rotary_dim;
+};
+constexpr int DA_WARPS = 4, DA_KEYS = 4, DA_STAGES = 3, DA_STAGE = 2 * DA_KEYS * 512 * DA_WARPS, DA_SMEM = DA_STAGES * DA_STAGE;
+constexpr float DA_LOG2E = 1.4426950408889634f;
+
+// 16 bytes into shared memory, or zeros where `live` is false (the address must be valid either way)
+__device__ __forceinline__ void cp_piece(uint32_t dst, const void* src, bool live) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ uint4 ld_piece(uint32_t at) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at) : "memory");
+  return v;
+}
+template <typename T> __device__ __forceinline__ void dec_unpack(const uint4& v, float (&f)[8]) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 t = DCvt<T>::to2(w[j]);
+    f[2 * j] = t.x; f[2 * j + 1] = t.y;
+  }
+}
+// eight dims from d0 on of a new q or k: rotated and rounded to T, as rotary_append_kernel stores them
+template <typename T> __device__ __forceinline__ uint4 dec_rotate(const uint4& raw, int d0, int rotary_dim, float pos, float log2_base) {
+  if (d0 >= rotary_dim) return raw;
+  float f[8];
+  dec_unpack<T>(raw, f);
+  uint4 out;
+  T* e = reinterpret_cast<T*>(&out);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int d = d0 + 2 * j;
+    if (d < rotary_dim) {
+      const float inv_freq = exp2f(-log2_base * static_cast<float>(d) / rotary_dim);
+      float sn, cs;
+      sincosf(pos * inv_freq, &sn, &cs);
+      e[2 * j] = DCvt<T>::from(f[2 * j] * cs - f[2 * j + 1] * sn);
+      e[2 * j + 1] = DCvt<T>::from(f[2 * j + 1] * cs + f[2 * j] * sn);
+    } else {
+      e[2 * j] = DCvt<T>::from(f[2 * j]);
+      e[2 * j + 1] = DCvt<T>::from(f[2 * j + 1]);
+    }
+  }
+  return out;
+}
+
+template <typename T, int LPK>
+__global__ void __launch_bounds__(DA_WARPS * 32, 4) decode_attn_kernel(const DecodeAttn p) {
+  constexpr int KPW = 32 / LPK, KB = DA_KEYS, DMAX = LPK * 8, BATCH = KB * KPW;
+  extern __shared__ __align__(16) unsigned char da_smem[];
+  __shared__ float red[DA_WARPS][DMAX];
+  __shared__ float stat[DA_WARPS][2];
+  __shared__ float fin[DMAX + 2];               // this split's output, maximum and sum
+  const int sp = blockIdx.x, h = blockIdx.y, b = blockIdx.z, D = p.D;
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, g = l / LPK, d0 = (l % LPK) * 8;
+  const bool act = d0 < D;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+  int len = p.lengths[b];
+  if (len < 0 || len > p.T) {                   // a length that does not fit the cache: never read past it
+    OSLO_REPORT_BOUNDS(p.err);
+    len = len < 0 ? 0 : p.T;
+  }
+  const int lo = p.window > 0 ? max(0, len - p.window) : 0;
+  const int span = len - lo, per = (span + p.splits - 1) / p.splits;
+  const int t0 = lo + sp * per, t1 = min(len, t0 + per);
+  const long long head = (static_cast<long long>(b) * p.H + h) * p.T * D;
+  const T* kb = reinterpret_cast<const T*>(p.kc) + head + d0;
+  const T* vb = reinterpret_cast<const T*>(p.vc) + head + d0;
+  int wi = -1;
+  if (p.k != nullptr) {
+    const long long at = p.write_index[0];
+    if (at < 0 || at >= p.T) OSLO_REPORT_BOUNDS(p.err);   // never write outside the cache
+    else wi = static_cast<int>(at);
+  }
+  const uint32_t ring = smem_u32(da_smem) + (w * (2 * KB * 32) + l) * 16;
+  int ft = t0 + w * BATCH, fslot = 0;
+  auto fetch = [&]() {
+    if (ft < t1) {
+      const uint32_t at = ring + fslot * DA_STAGE;
+#pragma unroll
+      for (int j = 0; j < KB; ++j) {
+        const int t = ft + j * KPW + g;
+        const bool in = act && t < t1 && t != wi;
+        const long long off = in ? static_cast<long long>(t) * D : -static_cast<long long>(d0);
+        cp_piece(at + j * 512, kb + off, in);
+        cp_piece(at + (KB + j) * 512, vb + off, in);
+      }
+    }
+    ft += DA_WARPS * BATCH;
+    if (++fslot == DA_STAGES) fslot = 0;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int i = 0; i < DA_STAGES - 1; ++i) fetch();
+
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  uint4 qraw = act ? *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.q) + b * p.q_sb + h * p.q_sh + d0) : zero;
+  uint4 knew = zero, vnew = zero;
+  if (p.k != nullptr) {
+    if (act) {
+      knew = *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.k) + b * p.k_sb + h * p.k_sh + d0);
+      vnew = *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.v) + b * p.v_sb + h * p.v_sh + d0);
+    }
+    if (p.rotary_dim > 0) {
+      const float pos = static_cast<float>(p.positions[b]);
+      qraw = dec_rotate<T>(qraw, d0, p.rotary_dim, pos, p.log2_base);
+      knew = dec_rotate<T>(knew, d0, p.rotary_dim, pos, p.log2_base);
+    }
+    if (wi >= 0 && sp == 0 && w == 0 && g == 0 && act) {
+      *reinterpret_cast<uint4*>(reinterpret_cast<T*>(p.kc) + head + static_cast<long long>(wi) * D + d0) = knew;
+      *reinterpret_cast<uint4*>(reinterpret_cast<T*>(p.vc) + head + static_cast<long long>(wi) * D + d0) = vnew;
+    }
+  }
+  float q[8];
+  dec_unpack<T>(qraw, q);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) q[i] *= p.scale * DA_LOG2E;
+  float m = -CUDART_INF_F, s = 0.f, acc[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+  int slot = 0;
+  for (int tb = t0 + w * BATCH; tb < t1; tb += DA_WARPS * BATCH) {
+    fetch();                                    // into the slot of the batch before this one
+    asm volatile("cp.async.wait_group %0;" ::"n"(DA_STAGES - 1) : "memory");
+    const uint32_t at = ring + slot * DA_STAGE;
+    if (++slot == DA_STAGES) slot = 0;
+    uint4 kr[KB], vr[KB];
+#pragma unroll
+    for (int j = 0; j < KB; ++j) {
+      kr[j] = ld_piece(at + j * 512);
+      vr[j] = ld_piece(at + (KB + j) * 512);
+    }
+    if (wi >= tb && wi < tb + BATCH) {          // the batch that the new token falls into
+#pragma unroll
+      for (int j = 0; j < KB; ++j)
+        if (tb + j * KPW + g == wi) { kr[j] = knew; vr[j] = vnew; }
+    }
+    float dot[KB];
+#pragma unroll
+    for (int j = 0; j < KB; ++j) {
+      float f[8], d = 0.f;
+      dec_unpack<T>(kr[j], f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) d += f[i] * q[i];
+      dot[j] = d;
+    }
+#pragma unroll
+    for (int off = LPK / 2; off > 0; off >>= 1) {
+#pragma unroll
+      for (int j = 0; j < KB; ++j) dot[j] += __shfl_xor_sync(0xffffffffu, dot[j], off);
+    }
+    float mn = m;
+#pragma unroll
+    for (int j = 0; j < KB; ++j) {
+      if (tb + j * KPW + g >= t1) dot[j] = -CUDART_INF_F;
+      mn = fmaxf(mn, dot[j]);
+    }
+    const float base = mn == -CUDART_INF_F ? 0.f : mn;   // this lane group may have no key in the batch
+    const float a = exp2f(m - base);
+    float ps = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] *= a;
+#pragma unroll
+    for (int j = 0; j < KB; ++j) {
+      const float pr = exp2f(dot[j] - base);
+      ps += pr;
+      float f[8];
+      dec_unpack<T>(vr[j], f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] += pr * f[i];
+    }
+    s = s * a + ps;
+    m = mn;
+  }
+  // the lane groups of a warp, the warps of the block, the splits of the cluster
+#pragma unroll
+  for (int off = LPK; off < 32; off <<= 1) {
+    const float mo = __shfl_xor_sync(0xffffffffu, m, off), so = __shfl_xor_sync(0xffffffffu, s, off);
+    const float mx = fmaxf(m, mo), base = mx == -CUDART_INF_F ? 0.f : mx;
+    const float a = exp2f(m - base), c = exp2f(mo - base);
+    s = s * a + so * c;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] = acc[i] * a + __shfl_xor_sync(0xffffffffu, acc[i], off) * c;
+    m = mx;
+  }
+  if (l == 0) { stat[w][0] = m; stat[w][1] = s; }
+  if (g == 0) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) red[w][d0 + i] = acc[i];
+  }
+  __syncthreads();
+  float gm = -CUDART_INF_F, gs = 0.f, wt[DA_WARPS];
+#pragma unroll
+  for (int i = 0; i < DA_WARPS; ++i) gm = fmaxf(gm, stat[i][0]);
+  {
+    const float base = gm == -CUDART_INF_F ? 0.f : gm;
+#pragma unroll
+    for (int i = 0; i < DA_WARPS; ++i) { wt[i] = exp2f(stat[i][0] - base); gs += stat[i][1] * wt[i]; }
+  }
+  T* o = reinterpret_cast<T*>(p.o) + (static_cast<long long>(b) * p.H + h) * D;
+  for (int d = threadIdx.x; d < DMAX; d += DA_WARPS * 32) {
+    float v = 0.f;
+#pragma unroll
+    for (int i = 0; i < DA_WARPS; ++i) v += red[i][d] * wt[i];
+    if (p.splits > 1) fin[d] = v;
+    else if (d < D) o[d] = DCvt<T>::from(gs > 0.f ? v / gs : (gs == gs ? 0.f : gs));
+  }
+  if (p.splits == 1) return;
+  if (threadIdx.x == 0) { fin[DMAX] = gm; fin[DMAX + 1] = gs; }
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  const int share = (D + p.splits - 1) / p.splits;
+  for (int dd = sp * share + threadIdx.x; dd < min(D, (sp + 1) * share); dd += DA_WARPS * 32) {
+    const uint32_t base = smem_u32(fin);
+    float pm[8], pv[8], psum[8], top = -CUDART_INF_F;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      if (r < p.splits) {
+        uint32_t peer;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(base), "r"(r));
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(pv[r]) : "r"(peer + dd * 4) : "memory");
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(pm[r]) : "r"(peer + DMAX * 4) : "memory");
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(psum[r]) : "r"(peer + (DMAX + 1) * 4) : "memory");
+      } else {
+        pv[r] = 0.f; pm[r] = -CUDART_INF_F; psum[r] = 0.f;
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 8; ++r) top = fmaxf(top, pm[r]);
+    const float ref = top == -CUDART_INF_F ? 0.f : top;
+    float tot = 0.f, out = 0.f;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const float c = exp2f(pm[r] - ref);
+      tot += psum[r] * c;
+      out += pv[r] * c;
+    }
+    o[dd] = DCvt<T>::from(tot > 0.f ? out / tot : (tot == tot ? 0.f : tot));
+  }
+  // no block leaves while another may still read its part
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <typename T, int LPK>
+static int decode_attn_launch(const DecodeAttn& p, int B, cudaStream_t st) {
+  cudaError_t e = cudaFuncSetAttribute(decode_attn_kernel<T, LPK>, cudaFuncAttributeMaxDynamicSharedMemorySize, DA_SMEM);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(p.splits, p.H, B);
+  cfg.blockDim = dim3(DA_WARPS * 32);
+  cfg.dynamicSmemBytes = DA_SMEM;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = p.splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, decode_attn_kernel<T, LPK>, p));
+}
+
 template <typename T>
-static int gemv_launch(const void* x1, int ld1, int K1, const void* x2, int ld2, int K2, const void* W, int ldw,
-                       const void* bias, const void* res, int ldr, void* out, int ldo, int M, int N, int gelu_from,
-                       int num_sms, cudaStream_t st, int parts = 1, long long sx = 0, long long sw = 0, long long so = 0) {
-  int blocks = N / GV_COLS;                   // one block per column group, at most 8 resident blocks per SM's worth
-  if (blocks > num_sms * 8 / parts) blocks = num_sms * 8 / parts;
-  if (blocks < 1) blocks = 1;
-#define GV_CASE(MR)                                                                                               \
-  gemv_rows_kernel<T, MR><<<dim3(blocks, parts), GV_THREADS, 0, st>>>((const T*)x1, ld1, K1, (const T*)x2, ld2, K2, (const T*)W, ldw, \
-                                                         (const T*)bias, (const T*)res, ldr, (T*)out, ldo, N, M, gelu_from, sx, sw, so)
-  if (M <= 1) GV_CASE(1);
-  else if (M <= 2) GV_CASE(2);
-  else GV_CASE(4);
-#undef GV_CASE
-  return static_cast<int>(cudaGetLastError());
+static int decode_attn_dispatch(const DecodeAttn& p, int B, cudaStream_t st) {
+  if (p.D <= 32) return decode_attn_launch<T, 4>(p, B, st);
+  if (p.D <= 64) return decode_attn_launch<T, 8>(p, B, st);
+  if (p.D <= 128) return decode_attn_launch<T, 16>(p, B, st);
+  return decode_attn_launch<T, 32>(p, B, st);
 }
 
 }  // namespace oslo
-
-extern "C" int oslo_gemv_rows(const void* x1, int ld1, int K1, const void* x2, int ld2, int K2, const void* W, int ldw,
-                              const void* bias, const void* res, int ldr, void* out, int ldo, int M, int N,
-                              int gelu_from, int dtype, int num_sms, cudaStream_t stream) {
-  using namespace oslo;
-  if (M <= 0 || N <= 0) return 0;
-  if (M > 4 || N % GV_COLS || K1 <= 0 || K1 % 8 || (x2 && (K2 <= 0 || K2 % 8)) || ld1 % 8 || ldw % 8 || (x2 && ld2 % 8))
-    return -1;
-  const void* ptrs[3] = {x1, x2, W};
-  for (const void* p : ptrs)
-    if (reinterpret_cast<uintptr_t>(p) & 15) return -4;
-  if (dtype == OSLO_DT_BF16)
-    return gemv_launch<__nv_bfloat16>(x1, ld1, K1, x2, ld2, x2 ? K2 : 0, W, ldw, bias, res, ldr, out, ldo, M, N, gelu_from, num_sms, stream);
-  if (dtype == OSLO_DT_FP16)
-    return gemv_launch<__half>(x1, ld1, K1, x2, ld2, x2 ? K2 : 0, W, ldw, bias, res, ldr, out, ldo, M, N, gelu_from, num_sms, stream);
-  return -2;
-}
-
-extern "C" int oslo_gemv_stacked(const void* x, int ldx, long long sx, const void* W, int ldw, long long sw, void* out, int P, int M,
-                                 int N, int K, int dtype, int num_sms, cudaStream_t stream) {
-  using namespace oslo;
-  if (P <= 0 || M <= 0 || N <= 0) return 0;
-  if (M > 4 || P > 64 || N % GV_COLS || K <= 0 || K % 8 || ldx % 8 || ldw % 8 || sx % 8 || sw % 8) return -1;
-  if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(W) & 15)) return -4;
-  const long long so = static_cast<long long>(M) * N;
-  if (dtype == OSLO_DT_BF16)
-    return gemv_launch<__nv_bfloat16>(x, ldx, K, nullptr, 0, 0, W, ldw, nullptr, nullptr, 0, out, N, M, N, -1, num_sms, stream, P, sx, sw, so);
-  if (dtype == OSLO_DT_FP16)
-    return gemv_launch<__half>(x, ldx, K, nullptr, 0, 0, W, ldw, nullptr, nullptr, 0, out, N, M, N, -1, num_sms, stream, P, sx, sw, so);
-  return -2;
-}
 
 extern "C" int oslo_rotary_append(const void* q, const void* k, const void* v, long long ldq, long long ldk,
                                   long long ldv, void* q_out, void* kc, void* vc, const int* lengths,
@@ -253,4 +375,35 @@ extern "C" int oslo_rotary_append(const void* q, const void* k, const void* v, l
   else
     return -2;
   return static_cast<int>(cudaGetLastError());
+}
+
+extern "C" int oslo_decode_attn(const void* q, const void* k, const void* v, void* kc, void* vc, void* o, long long q_sb,
+                                long long q_sh, long long k_sb, long long k_sh, long long v_sb, long long v_sh, const int* lengths,
+                                const int* positions, const long long* write_index, int B, int H, int T, int D, int rotary_dim,
+                                float base, float scale, int window, int dtype, int num_sms, int* err_word, cudaStream_t st) {
+  using namespace oslo;
+  if (B <= 0 || H <= 0) return 0;
+  if (D % 8 || D > 256 || D <= 0 || rotary_dim % 2 || rotary_dim > D || B > 65535 || H > 65535) return -3;
+  const long long strides[6] = {q_sb, q_sh, k_sb, k_sh, v_sb, v_sh};
+  for (int i = 0; i < (k ? 6 : 2); ++i)
+    if (strides[i] % 8) return -1;
+  const void* ptrs[5] = {q, k, v, kc, vc};
+  for (const void* p : ptrs)
+    if (reinterpret_cast<uintptr_t>(p) & 15) return -4;
+  DecodeAttn p = {};
+  p.q = q; p.k = k; p.v = v; p.kc = kc; p.vc = vc; p.o = o; p.lengths = lengths; p.positions = positions;
+  p.write_index = write_index; p.err = err_word;
+  p.q_sb = q_sb; p.q_sh = q_sh; p.k_sb = k_sb; p.k_sh = k_sh; p.v_sb = v_sb; p.v_sh = v_sh;
+  p.scale = scale; p.log2_base = log2f(base); p.H = H; p.T = T; p.D = D; p.window = window; p.rotary_dim = k ? rotary_dim : 0;
+  // Up to eight blocks per SM, two waves of the four that fit (8 rows x 16 heads x 2048 keys of 128: 29.5 us, 30.5 with one wave, and
+  // 37 in blocks of eight warps with up to ten per SM; 32 x 16 x 1101 keys of 256: 105, 113, 111), clusters of at most eight, and no
+  // split of fewer than 64 keys. The kernel before (4 to 16 of 32 lanes idle for narrow heads, one load deep, rotary, append and the
+  // merge of the splits in kernels of their own) took 64.6 and 103.9 us for these.
+  const int reach = window > 0 && window < T ? window : T;
+  int splits = static_cast<int>(8ll * num_sms / (static_cast<long long>(B) * H));
+  if (splits > reach / 64) splits = reach / 64;
+  p.splits = splits < 1 ? 1 : (splits > 8 ? 8 : splits);
+  if (dtype == OSLO_DT_BF16) return decode_attn_dispatch<__nv_bfloat16>(p, B, st);
+  if (dtype == OSLO_DT_FP16) return decode_attn_dispatch<__half>(p, B, st);
+  return -2;
 }

@@ -176,6 +176,9 @@ __global__ void __launch_bounds__(LN_THREADS) layernorm_rows_fwd_kernel(const T*
   const int li = (warp % WPR) * 32 + lane, nvec = cols / V;
   const bool live = row < rows;
   const size_t at = static_cast<size_t>(live ? row : 0) * cols;
+  // a programmatic launch: the blocks are in place when the kernel before completes, and the next one's when these have started
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
   float f[VPL][V];
   float s = 0.f;
 #pragma unroll
@@ -762,23 +765,6 @@ __global__ void __launch_bounds__(256) sumsq_kernel(const T* __restrict__ x, flo
   if (threadIdx.x == 0) atomicAdd(out, s);
 }
 
-// ---------------------------------------------------------------------- split-K GEMM finalisation
-// out[r, c] = T(act(sum_s ws[s, r, c] + bias[c])): sums the k-slice planes of a split-K GEMM in a fixed order
-template <typename T>
-__global__ void splitk_finalize_kernel(const float* __restrict__ ws, const T* __restrict__ bias, T* __restrict__ out,
-                                       long long n, int cols, int split_k, int gelu_from) {
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    float v = 0.f;
-    for (int s = 0; s < split_k; ++s) v += ws[s * n + i];
-    const int c = static_cast<int>(i % cols);
-    if (bias) v += Cvt<T>::to(bias[c]);
-    if (gelu_from >= 0 && c >= gelu_from) v = gelu_f(v);
-    if (gelu_from == OSLO_ACT_RELU2) { v = fmaxf(v, 0.f); v *= v; }
-    out[i] = Cvt<T>::from(v);
-  }
-}
-
 // ---------------------------------------------------------------------- n-gram blocking
 // thread `c` compares the (n-1)-gram starting at c with the last (n-1) tokens of the row; on a match the
 // token that followed it is banned. No shared memory is used, so the row length is unbounded.
@@ -828,8 +814,9 @@ using namespace oslo;
   else CALL(4, 8)
 
 #define LN_FWD(VPL, WPR)                                                                                        \
-  { layernorm_rows_fwd_kernel<T, VPL, WPR><<<(rows + 8 / WPR - 1) / (8 / WPR), LN_THREADS, 0, st>>>(             \
-        (const T*)x, (const T*)w, (const T*)b, (T*)y, mean, rstd, rows, cols, eps); }
+  { cfg.gridDim = dim3((rows + 8 / WPR - 1) / (8 / WPR));                                                          \
+    cudaLaunchKernelEx(&cfg, layernorm_rows_fwd_kernel<T, VPL, WPR>, (const T*)x, (const T*)w, (const T*)b, (T*)y, mean, rstd, rows, \
+                       cols, eps); }
 extern "C" int oslo_layernorm_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd,
                                   int rows, int cols, float eps, int dtype, cudaStream_t st) {
   if (rows <= 0) return 0;
@@ -840,6 +827,14 @@ extern "C" int oslo_layernorm_fwd(const void* x, const void* w, const void* b, v
       layernorm_fwd_kernel<T><<<rows, LN_THREADS, 0, st>>>((const T*)x, (const T*)w, (const T*)b, (T*)y, mean, rstd,
                                                            rows, cols, eps);
     } else {
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[0].val.programmaticStreamSerializationAllowed = 1;
+      cfg.blockDim = dim3(LN_THREADS);
+      cfg.stream = st;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
       LN_LAYOUT(nvec, LN_FWD)
     }
   })
@@ -1038,18 +1033,5 @@ extern "C" int oslo_ngram_ban(const long long* tokens, float* lprobs, int rows, 
                               int* err_word, cudaStream_t st) {
   if (rows == 0 || n <= 0 || len + 1 < n) return 0;
   ngram_ban_kernel<<<rows, 256, 0, st>>>(tokens, lprobs, len, vocab, n, err_word);
-  RET_LAST();
-}
-
-extern "C" int oslo_splitk_finalize(const float* ws, const void* bias, void* out, long long rows, int cols, int split_k,
-                                    int gelu_from, int dtype, cudaStream_t st) {
-  const long long n = rows * cols;
-  if (n == 0) return 0;
-  if (dtype == OSLO_DT_BF16)
-    splitk_finalize_kernel<__nv_bfloat16><<<grid_for(n, 256), 256, 0, st>>>(ws, (const __nv_bfloat16*)bias, (__nv_bfloat16*)out, n, cols, split_k, gelu_from);
-  else if (dtype == OSLO_DT_FP16)
-    splitk_finalize_kernel<__half><<<grid_for(n, 256), 256, 0, st>>>(ws, (const __half*)bias, (__half*)out, n, cols, split_k, gelu_from);
-  else
-    return -2;
   RET_LAST();
 }

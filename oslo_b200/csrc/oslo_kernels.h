@@ -45,17 +45,6 @@ int oslo_gemm_ce_16bit(const void* A, const void* B, int M, int N, int K, int ld
 int oslo_ce_reduce_stats(const float* stats, float* rowmax, float* sumexp, float* target, int rows, int blocks,
                          cudaStream_t stream);
 
-// few-row GEMM for decode steps (M <= 128): k range cut into `split_k` slices, slice s writes its fp32 partial sums
-// to plane s of D [split_k, M, N]; oslo_gemm_split_k_for suggests the slice count (1 = use oslo_gemm_16bit)
-int oslo_gemm_split_k_for(int M, int N, int K, int num_sms);
-int oslo_gemm_splitk_16bit(const void* A, const void* B, float* D, int M, int N, int K, int lda, int ldb, int ldd,
-                           int a_mn_major, int b_mn_major, int fp16, int split_k, int* err_word, int num_sms,
-                           cudaStream_t stream);
-// out = T(act(sum over planes of ws + bias)) for the [split_k, rows, cols] fp32 result of the split-K GEMM;
-// tanh-GeLU on columns >= gelu_from (-1 = none)
-int oslo_splitk_finalize(const float* ws, const void* bias, void* out, long long rows, int cols, int split_k,
-                         int gelu_from, int dtype, cudaStream_t stream);
-
 // LayerNorm over the last dim of [rows, cols]; mean/rstd are fp32 [rows]
 int oslo_layernorm_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd, int rows,
                        int cols, float eps, int dtype, cudaStream_t stream);
@@ -149,10 +138,12 @@ int oslo_flash_bwd_sm100(const void* q, const void* k, const void* v, const void
                          long long k_ss, long long v_sb, long long v_sh, long long v_ss, long long o_sb, long long o_sh,
                          long long o_ss, long long do_sb, long long do_sh, long long do_ss, float scale, int causal,
                          int window, int dtype, int* err_word, cudaStream_t stream);
-// single-query attention over a static cache [B, H, T, D]; lengths int32 [B]
-int oslo_decode_attn(const void* q, const void* kc, const void* vc, void* o, const int* lengths, float* ws, int B,
-                     int H, int T, int D, int splits, float scale, int window, int dtype, int* err_word,
-                     cudaStream_t stream);
+// single-query attention over a static cache [B, H, T, D]; lengths int32 [B]. q (and k, v of the new token, or null) [B, H, D] by the
+// strides of b and h; with k: rotary of the first rotary_dim dims at positions[b], k and v written at write_index[0] (decode_sm100.cu)
+int oslo_decode_attn(const void* q, const void* k, const void* v, void* kc, void* vc, void* o, long long q_sb, long long q_sh,
+                     long long k_sb, long long k_sh, long long v_sb, long long v_sh, const int* lengths, const int* positions,
+                     const long long* write_index, int B, int H, int T, int D, int rotary_dim, float base, float scale, int window,
+                     int dtype, int num_sms, int* err_word, cudaStream_t stream);
 
 // GEMM fused with a tensor-parallel collective (fused_comm_gemm.cu); mode 1 = all-reduce (result left in the
 // symmetric staging matrix), 2 = reduce-scatter into out, 3 = all-gather of A then GEMM into out
@@ -185,15 +176,16 @@ int oslo_ce_combine(const float* mx, const float* se, const float* tg, float* ou
                     void* const* peer_ptrs_dev, uint32_t* const* signal_ptrs_dev, uint32_t* counters, int n, int cap,
                     int rank, int world, int* err_word, cudaStream_t stream);
 
-// decode-step kernels (decode_sm100.cu). gemv_rows: out[m, n] = act([x1 | x2][m, :] . W[n, :] + bias[n]) for M <= 4
-// rows, W [N, K1 + K2] K-major, tanh-GeLU on columns >= gelu_from (-1 = none); x2 may be null.
-// `res` [M, N] (row stride ldr) is added after the activation; bias and res may be null.
-// P of them at once: x [P, M, K] and W [P, N, K] (strides sx, sw between parts) -> out [P, M, N]
-int oslo_gemv_stacked(const void* x, int ldx, long long sx, const void* W, int ldw, long long sw, void* out, int P, int M, int N, int K,
-                      int dtype, int num_sms, cudaStream_t stream);
-int oslo_gemv_rows(const void* x1, int ld1, int K1, const void* x2, int ld2, int K2, const void* W, int ldw,
-                   const void* bias, const void* res, int ldr, void* out, int ldo, int M, int N, int gelu_from,
-                   int dtype, int num_sms, cudaStream_t stream);
+// Products of at most 64 rows (few_rows_sm100.cu): out[m, n] = act([x1 | x2][m, :] . W[n, :] + bias[n]) + res[m, n], tanh-GeLU on
+// columns >= gelu_from (-1: none, OSLO_ACT_RELU2: square of relu); W = `parts` matrices [N / parts, K1 + K2] one below the other, or
+// with w_kn one [K1 + K2, N], N % 8 == 0. x2, bias, res may be null. With ln_w (M <= 8, M * K1 <= 8192, no x2): LayerNorm(x1) takes the
+// place of x1. More than 8 rows: K1 % 64 == 0 if there is an x2, (N / parts) % 128 == 0 if there are several weights.
+int oslo_few_rows(const void* x1, int ld1, int K1, const void* x2, int ld2, int K2, const void* w0, const void* w1, const void* w2,
+                  int parts, int ldw, int w_kn, const void* bias, const void* res, int ldr, const void* ln_w, const void* ln_b,
+                  float eps, void* out, int ldo, int M, int N, int gelu_from, int dtype, int* err_word, int num_sms, cudaStream_t stream);
+// P of them (M <= 8) at once: x [P, M, K] and W [P, N, K] (strides sx, sw between parts) -> out [P, M, N]
+int oslo_few_rows_stacked(const void* x, int ldx, long long sx, const void* W, int ldw, long long sw, void* out, int P, int M, int N,
+                          int K, int dtype, int num_sms, cudaStream_t stream);
 // rotary on the new token's q and k, q -> q_out [B, H, D], k / v -> cache [B, H, Tmax, D] at write_index[0];
 // the rotary position of row b is lengths[b]
 int oslo_rotary_append(const void* q, const void* k, const void* v, long long ldq, long long ldk, long long ldv,

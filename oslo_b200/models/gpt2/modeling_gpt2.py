@@ -22,7 +22,7 @@ from ...modeling_utils import (GPT2DoubleHeadsModelOutput, PretrainedConfig, Pre
 from ...parallel.layers import Conv1D, Embedding, LayerNorm, Linear
 from ...parallel.mpu import Layer, LayerPolicy
 from ..common import (AttentionCore, CausalLMHeadMixin, DecoderBackbone, SequenceClassificationMixin,
-                      maybe_dropout, merge_heads, split_heads, to_batch_seq, to_token_rows)
+                      decode_block, maybe_dropout, merge_heads, split_heads, to_batch_seq, to_token_rows)
 
 
 class GPT2Config(PretrainedConfig):
@@ -165,6 +165,11 @@ class GPT2Block(nn.Module):
         self.mlp = GPT2MLP(inner, config)
 
     def forward(self, hidden_states: Tensor, encoder_hidden_states=None, encoder_attention_mask=None, **kw):
+        if encoder_hidden_states is None and kw.get("cache") is not None:
+            attn, mlp = self.attn, self.mlp
+            fast = decode_block(self, attn, mlp, (attn.c_attn,), attn.c_proj, mlp.c_fc, mlp.c_proj, hidden_states, kw)
+            if fast is not None:
+                return fast, None, None
         a, present, probs = self.attn(self.ln_1(hidden_states), **kw)
         hidden_states = a + hidden_states
         if encoder_hidden_states is not None:

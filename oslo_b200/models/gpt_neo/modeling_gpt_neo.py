@@ -18,7 +18,7 @@ from ...modeling_utils import PretrainedConfig, PreTrainedModel
 from ...parallel.layers import Embedding, LayerNorm, Linear
 from ...parallel.mpu import Layer, LayerPolicy
 from ..common import (AttentionCore, CausalLMHeadMixin, DecoderBackbone, SequenceClassificationMixin,
-                      maybe_dropout, merge_heads, split_heads, to_batch_seq, to_token_rows)
+                      decode_block, maybe_dropout, merge_heads, split_heads, to_batch_seq, to_token_rows, unhooked)
 
 
 class GPTNeoConfig(PretrainedConfig):
@@ -149,6 +149,12 @@ class GPTNeoBlock(nn.Module):
         self.mlp = GPTNeoMLP(inner, config)
 
     def forward(self, hidden_states: Tensor, **kw):
+        if kw.get("cache") is not None and unhooked(self.attn):
+            attn, mlp = self.attn.attention, self.mlp
+            fast = decode_block(self, attn, mlp, (attn.q_proj, attn.k_proj, attn.v_proj), attn.out_proj, mlp.c_fc, mlp.c_proj,
+                                hidden_states, kw)
+            if fast is not None:
+                return fast, None, None
         a, present, probs = self.attn(self.ln_1(hidden_states), **kw)
         hidden_states = a + hidden_states
         hidden_states = hidden_states + self.mlp(self.ln_2(hidden_states))

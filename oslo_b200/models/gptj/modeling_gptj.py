@@ -20,7 +20,7 @@ from ...modeling_utils import PretrainedConfig, PreTrainedModel
 from ...parallel.layers import Embedding, LayerNorm, Linear, RowParallelLinear
 from ...parallel.mpu import Layer, LayerPolicy
 from ..common import (AttentionCore, CausalLMHeadMixin, DecoderBackbone, SequenceClassificationMixin,
-                      maybe_dropout, merge_heads, to_token_rows)
+                      maybe_dropout, merge_heads, to_token_rows, unhooked)
 
 
 def fixed_pos_embedding(x: Tensor, seq_dim: int = 1, seq_len: Optional[int] = None):
@@ -182,10 +182,11 @@ class GPTJBlock(nn.Module):
         self.attn = GPTJAttention(config)
         self.mlp = GPTJMLP(inner, config)
 
-    def _packed_decode_projections(self, x: Tensor):
+    def _packed_decode_projections(self, x: Tensor, ln: Optional[LayerNorm] = None):
         """Decode steps (few rows, no grad, fused kernels): q, k, v and fc_in + GeLU read the same LayerNorm output,
         so they run as ONE weight-streaming GEMM over a packed copy of the four weights (rebuilt when any of them
-        changes). Returns ``(q, k, v, h)`` or ``None`` when the ordinary per-layer path applies."""
+        changes). Returns ``(q, k, v, h)`` or ``None`` when the ordinary per-layer path applies. ``ln``: the LayerNorm
+        that is still to be applied to ``x``."""
         from ...config import get_config
         from ...ops import cuda_ops
         attn, mlp = self.attn, self.mlp
@@ -207,14 +208,23 @@ class GPTJBlock(nn.Module):
             self._packed_b = (torch.cat([fb.new_zeros(n_qkv), fb.detach()]) if fb is not None else None)
             self._packed_key = key
             self._packed_sizes = [w.size(0) for w in ws]
-        y = cuda_ops.packed_linear_small_m(x, self._packed_w, self._packed_b, sum(self._packed_sizes[:3]))
+        y = cuda_ops.few_rows(x, [self._packed_w], self._packed_b, sum(self._packed_sizes[:3]), ln=ln)
         return torch.split(y, self._packed_sizes, dim=-1)
 
-    def _decode_step(self, hidden_states: Tensor, x: Tensor, packed, kw):
-        """Whole block for one new token per row on a device-positioned static cache, in six launches: (LayerNorm and
-        the packed q/k/v/fc_in GEMV already done) rotary + cache append, decode attention (2), ONE GEMV for
-        out_proj and fc_out over [attention | mlp activation] - their sum is what the parallel residual needs -
-        ONE all-reduce under tensor parallelism instead of two, and the residual add. Returns ``None`` when the
+    def _fold_ln(self, hidden_states: Tensor) -> bool:
+        """Whether ``ln_1`` of these few rows is computed inside the packed projection's kernel."""
+        from ...ops import cuda_ops
+        ln = self.ln_1
+        return (hidden_states.is_cuda and type(ln) is LayerNorm and ln.oslo_fused and ln.weight is not None and unhooked(ln)
+                and cuda_ops.folded_ln_ok(hidden_states) and ln.weight.dtype == hidden_states.dtype
+                and ln.weight.numel() == hidden_states.size(-1)
+                and not (torch.is_grad_enabled() and (ln.weight.requires_grad or hidden_states.requires_grad)))
+
+    def _decode_step(self, hidden_states: Tensor, packed, kw):
+        """Whole block for one new token per row on a device-positioned static cache, in three launches: (LayerNorm and
+        the packed q/k/v/fc_in product already done) rotary, cache append and attention, ONE product for
+        out_proj and fc_out over [attention | mlp activation] with the residual - their sum is what the parallel
+        residual needs -, and ONE all-reduce under tensor parallelism instead of two. Returns ``None`` when the
         general path has to run."""
         from ...ops import cuda_ops
         attn, mlp = self.attn, self.mlp
@@ -237,27 +247,19 @@ class GPTJBlock(nn.Module):
         layer = kw["layer_id"]
         kc, vc = cache.k[layer], cache.v[layer]
         rd = attn.rotary_dim if attn.rotary_dim is not None else attn.head_dim
-        q_rot = cuda_ops.rotary_append(q, k, v, kc, vc, cache.lengths_dev, cache.write_index, rd)
-        o = ops.decode_attention(q_rot, kc, vc, cache.lengths_next, attn.scale, attn.window)
+        q, k, v = (t.unflatten(1, (kc.size(1), kc.size(3))) for t in (q, k, v))
+        o = cuda_ops.decode_step_attention(q, k, v, kc, vc, cache.lengths_next, cache.lengths_dev, cache.write_index,
+                                           attn.scale, attn.window, rd)
         mpu = getattr(attn.out_proj, "mpu", None)
         tp = mpu.tp if mpu is not None else 1
         fc_bias = mlp.fc_out.bias
-        if rows <= cuda_ops.GEMV_ROWS:
-            # bias and residual enter the sum exactly once: on tensor-parallel rank 0, before the all-reduce
-            first = tp == 1 or mpu.tp_rank == 0
-            z = cuda_ops.gemv_two_inputs(o.reshape(rows, -1), h, self._packed2_w, fc_bias if first else None,
-                                         hidden_states.reshape(rows, -1) if first else None)
-            if tp > 1:
-                z = mpu._reduce(z)
-            return z.view_as(hidden_states), None, None
-        # more rows than the CUDA cores can feed from HBM: tensor-core split-k GEMM over the joined input
-        z = cuda_ops.packed_linear_small_m(torch.cat([o.reshape(rows, -1), h], dim=1), self._packed2_w, None, -1)
+        # bias and residual enter the sum exactly once: on tensor-parallel rank 0, before the all-reduce
+        first = tp == 1 or mpu.tp_rank == 0
+        z = cuda_ops.gemv_two_inputs(o.reshape(rows, -1), h, self._packed2_w, fc_bias if first else None,
+                                     hidden_states.reshape(rows, -1) if first else None)
         if tp > 1:
             z = mpu._reduce(z)
-        z = z.view_as(hidden_states)
-        if fc_bias is not None:
-            z = z + fc_bias
-        return z + hidden_states, None, None
+        return z.view_as(hidden_states), None, None
 
     def _tp_shared_input(self, x: Tensor):
         """``(q, k, v, h)`` through ``fused_tp.tp_block_input`` when the four layers are plain column-parallel shards
@@ -285,10 +287,13 @@ class GPTJBlock(nn.Module):
                               mlp.fc_in.bias, attn.q_proj.mpu)
 
     def forward(self, hidden_states: Tensor, **kw):
-        x = self.ln_1(hidden_states)
-        packed = self._packed_decode_projections(x) if x.is_cuda else None
+        fold = hidden_states.is_cuda and self._fold_ln(hidden_states)
+        packed = self._packed_decode_projections(hidden_states, self.ln_1) if fold else None
+        x = hidden_states if packed is not None else self.ln_1(hidden_states)
+        if packed is None and x.is_cuda and not fold:
+            packed = self._packed_decode_projections(x)
         if packed is not None:
-            fast = self._decode_step(hidden_states, x, packed, kw)
+            fast = self._decode_step(hidden_states, packed, kw)
             if fast is not None:
                 return fast
             a, present, probs = self.attn(x, qkv=packed[:3], **kw)

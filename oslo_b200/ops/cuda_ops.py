@@ -104,8 +104,13 @@ def gemm_tn(d: Tensor, x: Tensor, out_dtype=None) -> Tensor:
     return gemm(d, x, True, True, flags=FLAG_OUT_FP32 if out_dtype == torch.float32 else 0)
 
 
-SMALL_M_ROWS = 64  # inference calls with at most this many rows use the split-K path
-GEMV_ROWS = 4      # ... and with at most this many rows the CUDA-core weight-streaming kernel
+SMALL_M_ROWS = 64  # inference calls with at most this many rows use the weight-streaming kernel
+STACKED_ROWS = 8   # rows of several stacked products that run in one launch of it
+
+
+def folded_ln_ok(x: Tensor) -> bool:
+    """Whether the weight-streaming kernel takes the LayerNorm of ``x`` along: every block computes it for itself."""
+    return x.numel() <= 8192 and x.numel() <= 8 * x.size(-1)
 
 
 def weight_grad(weight: Tensor, a: Tensor, b: Tensor) -> Optional[Tensor]:
@@ -297,30 +302,56 @@ def linear(x: Tensor, weight: Tensor, bias: Optional[Tensor], reversed_: bool, a
                and (bias is None or bias.dtype == x.dtype))
         if big:
             return _Linear.apply(x, weight, bias, reversed_, False, residual)
-        return linear(x, weight, bias, reversed_, activation) + residual
+        if (residual.shape != x.shape[:-1] + (n_,) or residual.dtype != x.dtype or not x.is_cuda
+                or (torch.is_grad_enabled() and residual.requires_grad) or not small_rows_ok(x, weight, bias, reversed_)):
+            return linear(x, weight, bias, reversed_, activation) + residual
     if activation is not None and activation not in _GELU + ("relu2",):
         raise ValueError(f"unsupported fused activation {activation!r}")
     n = weight.size(1) if reversed_ else weight.size(0)
     ok = (x.dtype in _16BIT and weight.dtype == x.dtype and x.size(-1) % 8 == 0 and n % 8 == 0 and x.numel() > 0
           and (bias is None or bias.dtype == x.dtype))
+    if small_rows_ok(x, weight, bias, reversed_):
+        gelu_from = -1 if activation is None else (ACT_RELU2 if activation == "relu2" else 0)
+        return few_rows(x, [weight], bias, gelu_from, residual, reversed_)
     if not ok:  # fp32 or ragged shapes: library GEMM, same semantics
         return ref.linear(x, weight, bias, reversed_, activation)
     rows = x.numel() // x.size(-1)
-    if rows <= SMALL_M_ROWS and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad)):
-        # decode steps: weight-streaming split-K GEMM so that every SM pulls weights, not just N / 128 of them
-        x2 = _as_operand(x.reshape(rows, x.size(-1)))
-        gelu_from = -1 if activation is None else (ACT_RELU2 if activation == "relu2" else 0)
-        if rows <= GEMV_ROWS and not reversed_ and n % 4 == 0:
-            y = _ext().gemv_rows(x2, None, _as_operand(weight), bias, gelu_from)   # no tensor-core tile to pad
-        else:
-            y = _ext().gemm_small_m(x2, _as_operand(weight), int(reversed_), bias, gelu_from)
-        return y.view(*x.shape[:-1], n)
     if activation == "relu2":
         if torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad):      # no backward of its own
             return torch.relu(_Linear.apply(x, weight, bias, reversed_, False, None)).pow(2)
         flags = FLAG_RELU2 | (FLAG_BIAS if bias is not None else 0)
         return gemm(x.reshape(rows, x.size(-1)), weight, False, reversed_, bias=bias, flags=flags).view(*x.shape[:-1], n)
     return _Linear.apply(x, weight, bias, reversed_, activation is not None, None)
+
+
+def small_rows_ok(x: Tensor, weight: Tensor, bias: Optional[Tensor], reversed_: bool) -> bool:
+    """Whether ``x W^T + b`` without gradients goes to the weight-streaming kernel: a few rows, k in 16-byte pieces, and any number of
+    columns for ``[out, in]`` weights (GPT-2's head of 50257 words: 23 us through the library's product, floor 12), a multiple of 8
+    for ``[in, out]``."""
+    if torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad):
+        return False
+    k = x.size(-1)
+    return (x.is_cuda and x.dtype in _16BIT and weight.dtype == x.dtype and k % 8 == 0 and 0 < x.numel() <= SMALL_M_ROWS * k
+            and weight.numel() > 0 and (not reversed_ or weight.size(1) % 8 == 0) and (bias is None or bias.dtype == x.dtype))
+
+
+def few_rows(x: Tensor, weights, bias: Optional[Tensor] = None, gelu_from: int = -1, residual: Optional[Tensor] = None,
+             reversed_: bool = False, ln=None) -> Tensor:
+    """``act(x W^T + bias) + residual`` of at most ``SMALL_M_ROWS`` rows; ``weights``: one matrix, or up to three ``[out, in]`` ones of
+    equal size side by side. ``ln`` (a LayerNorm module; see ``folded_ln_ok``): of ``ln(x)`` instead of ``x``."""
+    ws = [_as_operand(w) for w in weights]
+    if len({w.stride(0) for w in ws}) > 1:
+        ws = [w.contiguous() for w in ws]
+    k = x.size(-1)
+    y = _ext().few_rows(_as_operand(x.reshape(-1, k)), None, ws, int(reversed_), bias, int(gelu_from),
+                        None if residual is None else _rows_of(residual),
+                        None if ln is None else ln.weight, None if ln is None else ln.bias, 0.0 if ln is None else float(ln.eps))
+    return y.view(*x.shape[:-1], y.size(-1))
+
+
+def _rows_of(x: Tensor) -> Tensor:
+    x = x.reshape(-1, x.size(-1))
+    return x if x.stride(1) == 1 or x.size(1) == 1 else x.contiguous()
 
 
 def small_m_ok(x: Tensor, *weights: Tensor) -> bool:
@@ -332,23 +363,11 @@ def small_m_ok(x: Tensor, *weights: Tensor) -> bool:
             and all(w.dtype == x.dtype and w.size(0) % 8 == 0 for w in weights))
 
 
-def packed_linear_small_m(x: Tensor, weight: Tensor, bias: Optional[Tensor], gelu_from: int) -> Tensor:
-    """``x @ weight^T + bias`` for a few rows with tanh-GeLU on output columns ``>= gelu_from`` (-1: none);
-    ``weight`` is the row-wise concatenation of several ``[out_i, in]`` layers that share the input."""
-    rows = x.numel() // x.size(-1)
-    x2 = _as_operand(x.reshape(rows, x.size(-1)))
-    if rows <= GEMV_ROWS and weight.size(0) % 4 == 0:
-        y = _ext().gemv_rows(x2, None, _as_operand(weight), bias, int(gelu_from))
-    else:
-        y = _ext().gemm_small_m(x2, _as_operand(weight), 0, bias, int(gelu_from))
-    return y.view(*x.shape[:-1], weight.size(0))
-
-
 def gemv_two_inputs(x1: Tensor, x2: Tensor, weight: Tensor, bias: Optional[Tensor] = None,
                     residual: Optional[Tensor] = None) -> Tensor:
-    """``[x1 | x2] @ weight^T (+ bias) (+ residual)`` for at most ``GEMV_ROWS`` rows without materialising the
+    """``[x1 | x2] @ weight^T (+ bias) (+ residual)`` for at most ``SMALL_M_ROWS`` rows without materialising the
     concatenation."""
-    return _ext().gemv_rows(_as_operand(x1), _as_operand(x2), _as_operand(weight), bias, -1, residual)
+    return _ext().few_rows(_as_operand(x1), _as_operand(x2), [_as_operand(weight)], 0, bias, -1, residual)
 
 
 def rotary_append(q: Tensor, k: Tensor, v: Tensor, k_cache: Tensor, v_cache: Tensor, lengths: Tensor,
@@ -543,6 +562,27 @@ def decode_attention(q: Tensor, k_cache: Tensor, v_cache: Tensor, lengths: Tenso
     return _ext().decode_attn(q.contiguous(), k_cache, v_cache, lengths.to(torch.int32), float(scale), int(window or 0))
 
 
+def decode_step_ok(q: Tensor, k_cache: Tensor, v_cache: Tensor) -> bool:
+    """Whether the append (and rotary) of a new token runs inside the decode attention kernel; ``q``, ``k``, ``v``: ``[B, heads, D]``."""
+    return (q.is_cuda and q.dtype in _16BIT and k_cache.dtype == q.dtype and v_cache.dtype == q.dtype and k_cache.shape == v_cache.shape
+            and q.numel() > 0 and k_cache.size(0) == q.size(0) and q.size(-1) % 8 == 0 and q.size(-1) <= 256
+            and k_cache.is_contiguous() and v_cache.is_contiguous() and k_cache.data_ptr() % 16 == 0 and v_cache.data_ptr() % 16 == 0
+            and not (torch.is_grad_enabled() and q.requires_grad))
+
+
+def _heads16(x: Tensor) -> Tensor:
+    ok = x.stride(2) == 1 and x.stride(0) % 8 == 0 and x.stride(1) % 8 == 0 and x.data_ptr() % 16 == 0
+    return x if ok else x.contiguous()
+
+
+def decode_step_attention(q: Tensor, k: Tensor, v: Tensor, k_cache: Tensor, v_cache: Tensor, lengths: Tensor, positions: Tensor,
+                          write_index: Tensor, scale: float, window: Optional[int], rotary_dim: int = 0, base: float = 10000.0) -> Tensor:
+    """One new token per row: rotary on the first ``rotary_dim`` dims of ``q`` and ``k`` (at ``positions[b]``), ``k`` and ``v`` into the
+    caches at ``write_index[0]``, and attention of ``q`` over the first ``lengths[b]`` keys, the new one among them - one kernel."""
+    return _ext().decode_step_attn(_heads16(q), _heads16(k), _heads16(v), k_cache, v_cache, lengths, positions, write_index,
+                                   int(rotary_dim), float(base), float(scale), int(window or 0))
+
+
 class _CausalSoftmax(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, scale):
@@ -729,7 +769,7 @@ def stacked_linear(x: Tensor, weight: Tensor):
     n = weight.size(1)
     if not (gemm_ok(x[0], weight[0]) and n % 8 == 0):
         return torch.matmul(x, weight.transpose(1, 2)).unbind(0)
-    if rows <= GEMV_ROWS:
+    if rows <= STACKED_ROWS:
         return _ext().gemv_stacked(x, weight).unbind(0)
     if rows <= SMALL_M_ROWS and x.is_contiguous() and weight.is_contiguous():
         flat, w = x.view(parts * rows, k), weight.view(parts * n, k)

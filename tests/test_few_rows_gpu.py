@@ -1,0 +1,79 @@
+"""The decode step's kernels at the edges of their tiles: products of 1 to 64 rows, and attention that appends the new token itself."""
+import pytest
+import torch
+
+import oslo_b200 as ob
+
+pytestmark = pytest.mark.gpu
+EPS = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}
+
+
+def _close(y, ref, dtype):
+    """One rounding to 16 bits (half a unit of ``EPS`` per value) and 32-bit sums; the rest covers a row's GeLU by tanh.approx."""
+    assert torch.isfinite(y).all()
+    assert (y.double() - ref).norm() <= 1.5 * EPS[dtype] * ref.norm()
+    assert (y.double() - ref).abs().max() <= 4 * EPS[dtype] * ref.abs().max()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("kn", [False, True])
+@pytest.mark.parametrize("m", [1, 2, 3, 5, 8, 9, 16, 17, 31, 33, 64])
+@pytest.mark.parametrize("k1, k2, n", [(8, 0, 8), (40, 0, 72), (768, 0, 2304), (256, 1032, 264), (4104, 0, 1000), (64, 0, 50264)])
+def test_few_rows(dtype, kn, m, k1, k2, n):
+    from oslo_b200.ops import cuda_ops
+    ext = cuda_ops._ext()
+    torch.manual_seed(m * 7 + k1 + n)
+    mk = lambda *s: torch.randn(*s, device="cuda").to(dtype)  # noqa: E731
+    x1, x2, bias, res = mk(m, k1 + 8)[:, :k1], (mk(m, k2) if k2 else None), mk(n), mk(m, n)
+    w = mk(k1 + k2, n) if kn else mk(n, k1 + k2)
+    x = x1 if x2 is None else torch.cat([x1, x2], 1)
+    z = x.double() @ (w.double() if kn else w.double().t())
+    y = ext.few_rows(x1, x2, [w], int(kn), bias, n // 2, res)
+    z = z + bias.double()
+    z[:, n // 2:] = torch.nn.functional.gelu(z[:, n // 2:], approximate="tanh")
+    _close(y, z + res.double(), dtype)
+    if not kn and k2 == 0:
+        _close(ext.few_rows(x1, None, [w, w.flip(0).contiguous()], 0, None, -1), torch.cat([x1.double() @ w.double().t(), x1.double() @ w.flip(0).double().t()], 1), dtype)
+        odd = n - 3                                            # columns past the end belong to nobody
+        _close(ext.few_rows(x1, None, [w[:odd]], 0, bias[:odd], -1), x1.double() @ w[:odd].double().t() + bias[:odd].double(), dtype)
+    if m <= 8 and k2 == 0 and m * k1 <= 8192:
+        ln = torch.nn.LayerNorm(k1).to("cuda", dtype)
+        with torch.no_grad():
+            ln.weight.normal_(1, 0.1), ln.bias.normal_(0, 0.1)
+            h = torch.nn.functional.layer_norm(x1.double(), (k1,), ln.weight.double(), ln.bias.double(), ln.eps)
+            y = ext.few_rows(x1, None, [w], int(kn), None, -1, None, ln.weight, ln.bias, ln.eps)
+        # the normalised input is rounded to 16 bits, as the LayerNorm kernel rounds it
+        ref = h @ (w.double() if kn else w.double().t())
+        bound = 1.5 * EPS[dtype] * (h.norm() * w.double().norm() / (k1 * n) ** 0.5 * n ** 0.5 + ref.norm())
+        assert torch.isfinite(y).all() and (y.double() - ref).norm() <= bound
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("d, rotary", [(8, 0), (32, 8), (64, 0), (80, 32), (128, 64), (256, 64), (256, 0)])
+@pytest.mark.parametrize("b, h, t, at, window", [(1, 3, 1, 0, 0), (2, 12, 180, 173, 0), (8, 16, 512, 300, 0), (1, 16, 2048, 2047, 0), (3, 5, 700, 690, 256),
+                                                 (40, 16, 96, 33, 17)])
+def test_decode_step_attention(dtype, d, rotary, b, h, t, at, window):
+    """Append, rotary and attention in one kernel against the three separate statements."""
+    from oslo_b200.ops import cuda_ops
+    torch.manual_seed(d + t + b)
+    qkv = torch.randn(b, 3 * h * d + 8, device="cuda").to(dtype)
+    q, k, v = (qkv[:, i * h * d:(i + 1) * h * d].unflatten(1, (h, d)) for i in range(3))
+    kc, vc = (torch.randn(b, h, t, d, device="cuda").to(dtype) for _ in range(2))
+    kc[:, :, at:], vc[:, :, at:] = float("nan"), float("nan")   # what lies behind the new token is not read
+    lengths = torch.full((b,), at + 1, device="cuda", dtype=torch.int32)
+    index = torch.full((1,), at, device="cuda", dtype=torch.long)
+    k2, v2 = kc.clone(), vc.clone()
+    out = cuda_ops.decode_step_attention(q, k, v, k2, v2, lengths, lengths - 1, index, d ** -0.5, window or None, rotary)
+    if rotary:
+        pos = (lengths - 1).long()[:, None]
+        rot = lambda z: ob.ops.rotary_interleaved(z[:, None], pos, rotary)[:, 0]  # noqa: E731
+        q, k = rot(q), rot(k)
+    kc[:, :, at], vc[:, :, at] = k, v
+    tol = dict(atol=2 * EPS[dtype], rtol=4 * EPS[dtype])        # the prefill's rotary kernel may round the other way
+    torch.testing.assert_close(k2[:, :, :at + 1], kc[:, :, :at + 1], **tol)
+    assert torch.equal(v2[:, :, :at + 1], vc[:, :, :at + 1]) and torch.isnan(v2[:, :, at + 1:]).all()
+    lo = max(0, at + 1 - window) if window else 0
+    s = torch.einsum("bhd,bhtd->bht", q.double(), k2[:, :, lo:at + 1].double()) * d ** -0.5
+    ref = torch.einsum("bht,bhtd->bhd", s.softmax(-1), v2[:, :, lo:at + 1].double())
+    torch.testing.assert_close(out.double(), ref, atol=3 * EPS[dtype], rtol=3 * EPS[dtype])
+    torch.testing.assert_close(cuda_ops.decode_attention(q, k2, v2, lengths, d ** -0.5, window or None).double(), ref, atol=3 * EPS[dtype], rtol=3 * EPS[dtype])
