@@ -503,9 +503,20 @@ std::tuple<Tensor, Tensor, Tensor> flash_bwd(const Tensor& dout, const Tensor& q
   check_attn_operand(o, "o"); check_attn_operand(dout, "dout");
   c10::cuda::CUDAGuard guard(q.device());
   const int B = q.size(0), H = q.size(1), Sq = q.size(2), D = q.size(3), Sk = k.size(2);
-  Tensor dq = at::empty_strided(q.sizes(), q.strides(), q.options());
-  Tensor dk = at::empty_strided(k.sizes(), k.strides(), k.options());
-  Tensor dv = at::empty_strided(v.sizes(), v.strides(), v.options());
+  Tensor dq, dk, dv;
+  const int64_t W = q.size(1) * q.size(3);
+  const auto* qp = static_cast<const char*>(q.data_ptr());
+  if (k.sizes() == q.sizes() && v.sizes() == q.sizes() && k.strides() == q.strides() && v.strides() == q.strides() && q.stride(1) == D &&
+      q.stride(2) == 3 * W && q.stride(0) == q.size(2) * 3 * W && static_cast<const char*>(k.data_ptr()) == qp + W * q.element_size() &&
+      static_cast<const char*>(v.data_ptr()) == qp + 2 * W * q.element_size()) {
+    // slices of one projection's rows: their gradients are slices of one tensor too, so that nobody has to join them
+    Tensor all = at::empty({B, Sq, 3, H, D}, q.options()).permute({2, 0, 3, 1, 4});
+    dq = all[0]; dk = all[1]; dv = all[2];
+  } else {
+    dq = at::empty_strided(q.sizes(), q.strides(), q.options());
+    dk = at::empty_strided(k.sizes(), k.strides(), k.options());
+    dv = at::empty_strided(v.sizes(), v.strides(), v.options());
+  }
   Tensor delta = at::empty({B, H, Sq}, q.options().dtype(at::kFloat));
   const uint8_t* mp = (kpm.has_value() && kpm->defined()) ? kpm->data_ptr<uint8_t>() : nullptr;
   if (impl == 1) {
@@ -525,6 +536,20 @@ std::tuple<Tensor, Tensor, Tensor> flash_bwd(const Tensor& dout, const Tensor& q
                           dout.stride(1), dout.stride(2), static_cast<float>(scale), causal ? 1 : 0,
                           static_cast<int>(window), dt_code(q), cur_stream(D > 128 ? 4 : 3)), "flash_bwd");
   return {dq, dk, dv};
+}
+
+// k, v [B, H, S, D] (16-bit, contiguous D, 16-byte aligned rows) into positions start .. start + S of caches [B, H, T, D]
+void prompt_append(const Tensor& k, const Tensor& v, Tensor kc, Tensor vc, int64_t start) {
+  TORCH_CHECK(k.is_cuda() && k.dim() == 4 && k.sizes() == v.sizes() && k.stride(3) == 1 && v.stride(3) == 1 && k.element_size() == 2 &&
+                  v.scalar_type() == k.scalar_type() && v.device() == k.device(), "prompt_append: k and v");
+  TORCH_CHECK(kc.dim() == 4 && kc.is_contiguous() && vc.is_contiguous() && kc.sizes() == vc.sizes() && kc.size(0) == k.size(0) &&
+                  kc.size(1) == k.size(1) && kc.size(3) == k.size(3) && kc.scalar_type() == k.scalar_type() &&
+                  vc.scalar_type() == k.scalar_type() && kc.device() == k.device() && vc.device() == k.device(), "prompt_append: caches");
+  c10::cuda::CUDAGuard guard(k.device());
+  check_rc(oslo_prompt_append(k.data_ptr(), v.data_ptr(), kc.data_ptr(), vc.data_ptr(), k.stride(0), k.stride(1), k.stride(2), v.stride(0),
+                              v.stride(1), v.stride(2), static_cast<int>(k.size(0)), static_cast<int>(k.size(1)),
+                              static_cast<int>(k.size(2)), static_cast<int>(k.size(3)), static_cast<int>(kc.size(2)),
+                              static_cast<int>(start), cur_stream()), "prompt_append");
 }
 
 // q (and the new token's k, v) [B, H, D] with contiguous D; caches [B, H, T, D]. With k and v: rotary on q and k (rotary_dim > 0, at
@@ -1793,6 +1818,7 @@ TORCH_LIBRARY(oslo_b200, m) {
   m.def("gemm_comm(Tensor a, Tensor b, int a_mn, int b_mn, Tensor? bias, Tensor? aux, Tensor(a!)? aux_out, Tensor(b!)? out, int flags, float alpha, int M, int N, int K, int peer_bufs_dev, int own_buf, int mc_base, int data_off, int flag_off, int flag_bytes, int rank, int world, int epoch, int done_base, int mode, bool use_multimem, Tensor(c!)? trace) -> int");
   m.def("few_rows(Tensor x1, Tensor? x2, Tensor[] w, int w_kn, Tensor? bias, int gelu_from, Tensor? res=None, Tensor? ln_w=None, "
         "Tensor? ln_b=None, float eps=0.0) -> Tensor");
+  m.def("prompt_append(Tensor k, Tensor v, Tensor(a!) kc, Tensor(b!) vc, int start) -> ()");
   m.def("decode_step_attn(Tensor q, Tensor? k, Tensor? v, Tensor(a!) kc, Tensor(b!) vc, Tensor lengths, Tensor? positions, "
         "Tensor? write_index, int rotary_dim, float base, float scale, int window) -> Tensor");
   m.def("gemv_rows(Tensor x1, Tensor? x2, Tensor w, Tensor? bias, int gelu_from, Tensor? res=None) -> Tensor");
@@ -1870,6 +1896,7 @@ TORCH_LIBRARY_IMPL(oslo_b200, CUDA, m) {
   m.impl("decode_attn", &decode_attn);
   m.impl("gemm_comm", &gemm_comm);
   m.impl("few_rows", &few_rows);
+  m.impl("prompt_append", &prompt_append);
   m.impl("decode_step_attn", &decode_step_attn);
   m.impl("gemv_rows", &gemv_rows);
   m.impl("rotary_append", &rotary_append);

@@ -2,6 +2,7 @@
 // weight products are in few_rows_sm100.cu.
 //   * rotary_append_kernel: GPT-J rotary on q and k of the new token, q to a contiguous buffer, k and v written
 //     into the static cache at the position held in device memory.
+//   * prompt_append_kernel: the keys and values of a prompt into the cache.
 //   * decode_attn_kernel: attention of one query per row over the cache, with the rotary and the append of the new token inside
 //     when it is given one.
 //
@@ -66,6 +67,37 @@ __global__ void rotary_append_kernel(const T* __restrict__ q, const T* __restric
     qo[d0] = DCvt<T>::from(q0); qo[d0 + 1] = DCvt<T>::from(q1);
     ko[d0] = DCvt<T>::from(k0); ko[d0 + 1] = DCvt<T>::from(k1);
     vo[d0] = vp[d0]; vo[d0 + 1] = vp[d0 + 1];
+  }
+}
+
+// k, v [B, H, S, D] by strides -> cache[b, h, start + s, :], in 16-byte pieces, four in flight per thread. Bound by memory: the library's
+// strided copies moved 134 MB in 108 us each (4 x 16 x 2048 x 256, one tensor).
+template <typename V>
+__global__ void __launch_bounds__(256) prompt_append_kernel(const V* __restrict__ k, const V* __restrict__ v, V* __restrict__ kc, V* __restrict__ vc,
+                                                            long long k_sb, long long k_sh, long long k_ss, long long v_sb, long long v_sh,
+                                                            long long v_ss, int H, int S, int per, int T, int start, long long total) {
+  const long long step = static_cast<long long>(gridDim.x) * blockDim.x;
+  const V* src = blockIdx.y ? v : k;
+  V* dst = blockIdx.y ? vc : kc;
+  const long long sb = blockIdx.y ? v_sb : k_sb, sh = blockIdx.y ? v_sh : k_sh, ss = blockIdx.y ? v_ss : k_ss;
+  for (long long i0 = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i0 < total; i0 += 4 * step) {
+    V piece[4];
+    long long at[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long i = i0 + u * step;       // (b, s, h, piece): the order of a projection's rows
+      if (i >= total) continue;
+      const int c = static_cast<int>(i % per);
+      long long r = i / per;
+      const int h = static_cast<int>(r % H);
+      r /= H;
+      const int s = static_cast<int>(r % S), b = static_cast<int>(r / S);
+      piece[u] = src[b * sb + h * sh + s * ss + c];
+      at[u] = ((static_cast<long long>(b) * H + h) * T + start + s) * per + c;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i0 + u * step < total) dst[at[u]] = piece[u];
   }
 }
 
@@ -374,6 +406,27 @@ extern "C" int oslo_rotary_append(const void* q, const void* k, const void* v, l
                                                                write_index, H, D, Tmax, rotary_dim, log2f(base), err_word);
   else
     return -2;
+  return static_cast<int>(cudaGetLastError());
+}
+
+extern "C" int oslo_prompt_append(const void* k, const void* v, void* kc, void* vc, long long k_sb, long long k_sh, long long k_ss,
+                                  long long v_sb, long long v_sh, long long v_ss, int B, int H, int S, int D, int T, int start,
+                                  cudaStream_t st) {
+  using namespace oslo;
+  if (B <= 0 || H <= 0 || S <= 0 || D <= 0) return 0;
+  if (D % 8 || start < 0 || start + S > T) return -1;
+  const long long strides[6] = {k_sb, k_sh, k_ss, v_sb, v_sh, v_ss};
+  for (long long s : strides)
+    if (s % 8) return -1;
+  const void* ptrs[4] = {k, v, kc, vc};
+  for (const void* p : ptrs)
+    if (reinterpret_cast<uintptr_t>(p) & 15) return -4;
+  const int per = D / 8;
+  const long long total = static_cast<long long>(B) * H * S * per;
+  const long long blocks = (total + 1023) / 1024;
+  prompt_append_kernel<uint4><<<dim3(static_cast<unsigned>(blocks < 148 * 32 ? blocks : 148 * 32), 2), 256, 0, st>>>(
+      (const uint4*)k, (const uint4*)v, (uint4*)kc, (uint4*)vc, k_sb / 8, k_sh / 8, k_ss / 8, v_sb / 8, v_sh / 8, v_ss / 8, H, S, per, T,
+      start, total);
   return static_cast<int>(cudaGetLastError());
 }
 

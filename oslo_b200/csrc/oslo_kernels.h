@@ -138,6 +138,9 @@ int oslo_flash_bwd_sm100(const void* q, const void* k, const void* v, const void
                          long long k_ss, long long v_sb, long long v_sh, long long v_ss, long long o_sb, long long o_sh,
                          long long o_ss, long long do_sb, long long do_sh, long long do_ss, float scale, int causal,
                          int window, int dtype, int* err_word, cudaStream_t stream);
+// k, v [B, H, S, D] (strides of b, h, s; 16-bit elements) into cache positions start .. start + S (decode_sm100.cu)
+int oslo_prompt_append(const void* k, const void* v, void* kc, void* vc, long long k_sb, long long k_sh, long long k_ss, long long v_sb,
+                       long long v_sh, long long v_ss, int B, int H, int S, int D, int T, int start, cudaStream_t stream);
 // single-query attention over a static cache [B, H, T, D]; lengths int32 [B]. q (and k, v of the new token, or null) [B, H, D] by the
 // strides of b and h; with k: rotary of the first rotary_dim dims at positions[b], k and v written at write_index[0] (decode_sm100.cu)
 int oslo_decode_attn(const void* q, const void* k, const void* v, void* kc, void* vc, void* o, long long q_sb, long long q_sh,

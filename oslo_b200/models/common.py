@@ -118,6 +118,11 @@ class StaticKVCache:
             self.v[layer].index_copy_(2, self.write_index, v)
             # `end` is only right outside graph replay; the decode kernel reads the valid length from lengths_next
             return self.k[layer], self.v[layer], end
+        if k.is_cuda:
+            from ..ops import cuda_ops, use_kernels
+            if use_kernels(k) and cuda_ops.prompt_append_ok(k, v, self.k[layer], self.v[layer]):
+                cuda_ops.prompt_append(k, v, self.k[layer], self.v[layer], self.length)
+                return self.k[layer], self.v[layer], end
         self.k[layer][:, :, self.length:end].copy_(k)
         self.v[layer][:, :, self.length:end].copy_(v)
         return self.k[layer], self.v[layer], end
@@ -262,6 +267,22 @@ def unhooked(*modules: nn.Module) -> bool:
     """Whether a block may compute what these modules compute without calling them: nobody listens to their calls."""
     g = nn.modules.module
     return not (g._global_forward_hooks or g._global_forward_pre_hooks) and not any(m._forward_hooks or m._forward_pre_hooks for m in modules)
+
+
+def residual_inside(block, attn, mlp, out_proj, fc_in, fc_out, hidden_states: Tensor, kw) -> bool:
+    """Whether a pre-norm block's two residual additions run inside GEMM epilogues, and its MLP as one autograd node: plain fused layers
+    on a CUDA input of the large-input path, and no dropout in between."""
+    if not (hidden_states.is_cuda and attn.fused and mlp.fused and mlp.activation in GELU_TANH_NAMES and kw.get("seq_shape") is None
+            and type(out_proj) is type(fc_in) is type(fc_out) and not (block.training and (attn.resid_pdrop or mlp.resid_pdrop))):
+        return False
+    from ..config import get_config
+    from ..ops import cuda_ops
+    from ..parallel.layers import Conv1D, Linear
+    kind = type(fc_out)
+    return (kind in (Conv1D, Linear) and get_config().block_fusion and all(m.oslo_fused for m in (out_proj, fc_in, fc_out))
+            and unhooked(mlp, fc_in, fc_out)
+            and all(m.bias is None or m.bias.dtype == hidden_states.dtype for m in (fc_in, fc_out))
+            and cuda_ops.fused_mlp_ok(hidden_states, fc_in.weight, fc_out.weight, kind is Conv1D))
 
 
 def decode_block(block, attn, mlp, qkv, out_proj, fc_in, fc_out, hidden_states: Tensor, kw) -> Optional[Tensor]:

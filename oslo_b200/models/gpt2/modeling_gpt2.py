@@ -22,7 +22,7 @@ from ...modeling_utils import (GPT2DoubleHeadsModelOutput, PretrainedConfig, Pre
 from ...parallel.layers import Conv1D, Embedding, LayerNorm, Linear
 from ...parallel.mpu import Layer, LayerPolicy
 from ..common import (AttentionCore, CausalLMHeadMixin, DecoderBackbone, SequenceClassificationMixin,
-                      decode_block, maybe_dropout, merge_heads, split_heads, to_batch_seq, to_token_rows)
+                      decode_block, maybe_dropout, residual_inside, merge_heads, split_heads, to_batch_seq, to_token_rows)
 
 
 class GPT2Config(PretrainedConfig):
@@ -90,7 +90,7 @@ class GPT2Attention(AttentionCore):
 
     def forward(self, hidden_states: Tensor, layer_past=None, attention_mask=None, position_ids=None,
                 head_mask=None, use_cache=False, output_attentions=False, cache=None, layer_id=0,
-                encoder_hidden_states=None, encoder_attention_mask=None, seq_shape=None):
+                encoder_hidden_states=None, encoder_attention_mask=None, seq_shape=None, residual=None):
         nh, hd = self.num_heads, self.head_dim
         if encoder_hidden_states is not None:
             if not self.is_cross_attention:
@@ -101,12 +101,27 @@ class GPT2Attention(AttentionCore):
             out, probs = self._cross_attention(q, k, v, encoder_attention_mask, head_mask)
             present = None
         else:
-            q, k, v = to_batch_seq(self.c_attn(hidden_states), seq_shape).split(self.split_size, dim=2)
-            q, k, v = split_heads(q, nh, hd), split_heads(k, nh, hd), split_heads(v, nh, hd)
-            out, present, probs = self.attend_with_cache(q, k, v, layer_past, cache, layer_id, attention_mask,
-                                                         use_cache, output_attentions, head_mask)
+            qkv = to_batch_seq(self.c_attn(hidden_states), seq_shape)
+            if self._packed(qkv, layer_past, cache, use_cache, output_attentions, head_mask):
+                from ...ops import cuda_ops
+                out, present, probs = cuda_ops.packed_attention(qkv, nh, self.window, self.scale, attention_mask), None, None
+            else:
+                q, k, v = qkv.split(self.split_size, dim=2)
+                q, k, v = split_heads(q, nh, hd), split_heads(k, nh, hd), split_heads(v, nh, hd)
+                out, present, probs = self.attend_with_cache(q, k, v, layer_past, cache, layer_id, attention_mask,
+                                                             use_cache, output_attentions, head_mask)
+        if residual is not None:      # only offered by the block where no dropout follows
+            return self.c_proj(to_token_rows(merge_heads(out), seq_shape), residual=residual), present, probs
         out = self.c_proj(to_token_rows(merge_heads(out), seq_shape))
         return maybe_dropout(out, self.resid_pdrop, self.training), present, probs
+
+    def _packed(self, qkv: Tensor, layer_past, cache, use_cache, output_attentions, head_mask) -> bool:
+        """Whether attention takes the joint projection's rows as they are: training calls that keep no keys and values."""
+        if not (self.fused and qkv.is_cuda and qkv.requires_grad and layer_past is None and cache is None and not use_cache
+                and not output_attentions and head_mask is None and not (self.training and self.attn_pdrop > 0.0)):
+            return False
+        from ...ops import cuda_ops, use_kernels
+        return use_kernels(qkv) and cuda_ops.packed_attention_ok(qkv, self.num_heads)
 
     def _cross_attention(self, q, k, v, encoder_attention_mask, head_mask):
         """Non-causal attention over encoder states; padded keys get -10000 before the softmax."""
@@ -170,6 +185,13 @@ class GPT2Block(nn.Module):
             fast = decode_block(self, attn, mlp, (attn.c_attn,), attn.c_proj, mlp.c_fc, mlp.c_proj, hidden_states, kw)
             if fast is not None:
                 return fast, None, None
+        if encoder_hidden_states is None and residual_inside(self, self.attn, self.mlp, self.attn.c_proj, self.mlp.c_fc, self.mlp.c_proj,
+                                                             hidden_states, kw):
+            from ...ops import cuda_ops
+            mlp = self.mlp
+            hidden_states, present, probs = self.attn(self.ln_1(hidden_states), residual=hidden_states, **kw)
+            return cuda_ops.fused_mlp(self.ln_2(hidden_states), mlp.c_fc.weight, mlp.c_fc.bias, mlp.c_proj.weight, mlp.c_proj.bias,
+                                      hidden_states, True), present, probs
         a, present, probs = self.attn(self.ln_1(hidden_states), **kw)
         hidden_states = a + hidden_states
         if encoder_hidden_states is not None:

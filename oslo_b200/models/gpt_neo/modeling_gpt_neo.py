@@ -13,12 +13,13 @@ from typing import List
 import torch.nn as nn
 from torch import Tensor
 
+from ...config import get_config
 from ...fused_kernels_utils import ACT2FN, GELU_TANH_NAMES
 from ...modeling_utils import PretrainedConfig, PreTrainedModel
 from ...parallel.layers import Embedding, LayerNorm, Linear
 from ...parallel.mpu import Layer, LayerPolicy
 from ..common import (AttentionCore, CausalLMHeadMixin, DecoderBackbone, SequenceClassificationMixin,
-                      decode_block, maybe_dropout, merge_heads, split_heads, to_batch_seq, to_token_rows, unhooked)
+                      decode_block, maybe_dropout, residual_inside, merge_heads, split_heads, to_batch_seq, to_token_rows, unhooked)
 
 
 class GPTNeoConfig(PretrainedConfig):
@@ -76,15 +77,26 @@ class GPTNeoSelfAttention(AttentionCore):
         self.out_proj = Linear(self.embed_dim, self.embed_dim, bias=True)
 
     def forward(self, hidden_states: Tensor, layer_past=None, attention_mask=None, position_ids=None,
-                head_mask=None, use_cache=False, output_attentions=False, cache=None, layer_id=0, seq_shape=None):
+                head_mask=None, use_cache=False, output_attentions=False, cache=None, layer_id=0, seq_shape=None, residual=None):
         nh, hd = self.num_heads, self.head_dim
-        q = split_heads(to_batch_seq(self.q_proj(hidden_states), seq_shape), nh, hd)
-        k = split_heads(to_batch_seq(self.k_proj(hidden_states), seq_shape), nh, hd)
-        v = split_heads(to_batch_seq(self.v_proj(hidden_states), seq_shape), nh, hd)
+        q, k, v = (split_heads(to_batch_seq(t, seq_shape), nh, hd) for t in self._project(hidden_states))
         out, present, probs = self.attend_with_cache(q, k, v, layer_past, cache, layer_id, attention_mask,
                                                      use_cache, output_attentions, head_mask)
+        if residual is not None:      # only offered by the block where no dropout follows
+            return self.out_proj(to_token_rows(merge_heads(out), seq_shape), residual=residual), present, probs
         out = self.out_proj(to_token_rows(merge_heads(out), seq_shape))
         return maybe_dropout(out, self.resid_pdrop, self.training), present, probs
+
+    def _project(self, x: Tensor):
+        """q, k and v; as one autograd node (their input gradients accumulate inside the GEMM epilogues) where the layers are plain
+        fused ones on a CUDA input of the large-input path."""
+        layers = (self.q_proj, self.k_proj, self.v_proj)
+        if (self.fused and x.is_cuda and all(type(l) is Linear and l.oslo_fused and l.bias is None for l in layers)
+                and unhooked(*layers) and get_config().block_fusion):
+            from ...ops import cuda_ops
+            if cuda_ops.qkv_linear_ok(x, *(l.weight for l in layers)):
+                return cuda_ops.qkv_linear(x, *(l.weight for l in layers))
+        return tuple(l(x) for l in layers)
 
 
 class GPTNeoLocalSelfAttention(GPTNeoSelfAttention):
@@ -155,6 +167,12 @@ class GPTNeoBlock(nn.Module):
                                 hidden_states, kw)
             if fast is not None:
                 return fast, None, None
+        attn, mlp = self.attn.attention, self.mlp
+        if residual_inside(self, attn, mlp, attn.out_proj, mlp.c_fc, mlp.c_proj, hidden_states, kw):
+            from ...ops import cuda_ops
+            hidden_states, present, probs = self.attn(self.ln_1(hidden_states), residual=hidden_states, **kw)
+            return cuda_ops.fused_mlp(self.ln_2(hidden_states), mlp.c_fc.weight, mlp.c_fc.bias, mlp.c_proj.weight, mlp.c_proj.bias,
+                                      hidden_states), present, probs
         a, present, probs = self.attn(self.ln_1(hidden_states), **kw)
         hidden_states = a + hidden_states
         hidden_states = hidden_states + self.mlp(self.ln_2(hidden_states))

@@ -83,18 +83,22 @@ class GPTJAttention(AttentionCore):
                 qkv=None, residual=None, partial_only=False):
         b, s = seq_shape if seq_shape is not None else hidden_states.shape[:2]
         nh, hd = self.num_attention_heads, self.head_dim
+        own = False                      # q and k are fresh, nobody else's, and without gradients
         if qkv is not None:   # already projected by the block's packed decode GEMM
             q, k, v = (t.reshape(b, s, nh, hd) for t in qkv)
         elif self._one_node_qkv(hidden_states):
             from ...ops import cuda_ops
             q, k, v = (t.view(b, s, nh, hd) for t in cuda_ops.qkv_linear(
                 hidden_states, self.q_proj.weight, self.k_proj.weight, self.v_proj.weight))
+            own = not (q.requires_grad or k.requires_grad)
         else:
             q = self.q_proj(hidden_states).view(b, s, nh, hd)
             k = self.k_proj(hidden_states).view(b, s, nh, hd)
             v = self.v_proj(hidden_states).view(b, s, nh, hd)
         rd = self.rotary_dim if self.rotary_dim is not None else hd
         rot = ops.rotary_interleaved if self.fused else ops.reference.rotary_interleaved
+        if own and self.fused and ops.use_kernels(q):
+            rot = cuda_ops.rotary_own
         q, k = rot(q, position_ids, rd), rot(k, position_ids, rd)
         q, k, v = (t.permute(0, 2, 1, 3) for t in (q, k, v))
         out, present, probs = self.attend_with_cache(q, k, v, layer_past, cache, layer_id, attention_mask,

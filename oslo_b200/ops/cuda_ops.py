@@ -181,31 +181,32 @@ class _Linear(torch.autograd.Function):
 
 
 class _FusedMLP(torch.autograd.Function):
-    """``fc_out(gelu(fc_in(x)))`` for ``[out, in]`` weights. The backward multiplies by ``gelu'`` inside the epilogue
+    """``fc_out(gelu(fc_in(x)))`` for ``[out, in]`` weights (``reversed_``: ``[in, out]``). The backward multiplies by ``gelu'`` inside the epilogue
     of fc_out's input-gradient GEMM instead of running a separate pass over the ``[rows, 4 * hidden]`` activation
     gradient."""
 
     @staticmethod
-    def forward(ctx, x, w_in, b_in, w_out, b_out, residual=None):
+    def forward(ctx, x, w_in, b_in, w_out, b_out, residual=None, reversed_=False):
         k = x.size(-1)
+        inner, n = (w_in.size(1), w_out.size(1)) if reversed_ else (w_in.size(0), w_out.size(0))
         x2 = x.reshape(-1, k)
         need_grad = any(ctx.needs_input_grad)
         flags = FLAG_GELU | (FLAG_BIAS if b_in is not None else 0)
         z = None
         if need_grad:
             flags |= FLAG_SAVE_PREACT
-            z = torch.empty(x2.size(0), w_in.size(0), dtype=x.dtype, device=x.device)
-        h = gemm(x2, w_in, False, False, bias=b_in, aux_out=z, flags=flags)
-        y = torch.empty(*x.shape[:-1], w_out.size(0), dtype=x.dtype, device=x.device)
+            z = torch.empty(x2.size(0), inner, dtype=x.dtype, device=x.device)
+        h = gemm(x2, w_in, False, reversed_, bias=b_in, aux_out=z, flags=flags)
+        y = torch.empty(*x.shape[:-1], n, dtype=x.dtype, device=x.device)
         res2 = None
         if residual is not None:
-            res2 = residual.reshape(-1, w_out.size(0))
+            res2 = residual.reshape(-1, n)
             if res2.stride(-1) != 1:
                 res2 = res2.contiguous()
-        gemm(h, w_out, False, False, bias=b_out, aux=res2, out=y.view(-1, w_out.size(0)),
+        gemm(h, w_out, False, reversed_, bias=b_out, aux=res2, out=y.view(-1, n),
              flags=(FLAG_BIAS if b_out is not None else 0) | (FLAG_RESIDUAL if residual is not None else 0))
         ctx.save_for_backward(x2, w_in, w_out, z, h)
-        ctx.has_b_in, ctx.has_b_out, ctx.in_shape = b_in is not None, b_out is not None, x.shape
+        ctx.has_b_in, ctx.has_b_out, ctx.in_shape, ctx.reversed = b_in is not None, b_out is not None, x.shape, reversed_
         ctx.has_residual = residual is not None
         return y
 
@@ -217,31 +218,34 @@ class _FusedMLP(torch.autograd.Function):
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
         dx = dw_in = db_in = dw_out = db_out = None
-        dz = gemm(dy2, w_out, False, True, aux=z, flags=FLAG_DGELU)      # (dy W_out) * gelu'(z)
+        rev = ctx.reversed
+        dz = gemm(dy2, w_out, False, not rev, aux=z, flags=FLAG_DGELU)      # (dy W_out) * gelu'(z)
         if ctx.needs_input_grad[3]:
-            dw_out = weight_grad(w_out, dy2, h)
+            dw_out = weight_grad(w_out, h, dy2) if rev else weight_grad(w_out, dy2, h)
         if ctx.has_b_out and ctx.needs_input_grad[4]:
             db_out = ext.colsum(dy2).to(dy.dtype)
         if ctx.needs_input_grad[0]:
-            dx = gemm(dz, w_in, False, True).view(ctx.in_shape)
+            dx = gemm(dz, w_in, False, not rev).view(ctx.in_shape)
         if ctx.needs_input_grad[1]:
-            dw_in = weight_grad(w_in, dz, x2)
+            dw_in = weight_grad(w_in, x2, dz) if rev else weight_grad(w_in, dz, x2)
         if ctx.has_b_in and ctx.needs_input_grad[2]:
             db_in = ext.colsum(dz).to(dy.dtype)
         d_res = dy if (ctx.has_residual and ctx.needs_input_grad[5]) else None
-        return dx, dw_in, db_in, dw_out, db_out, d_res
+        return dx, dw_in, db_in, dw_out, db_out, d_res, None
 
 
-def fused_mlp_ok(x: Tensor, w_in: Tensor, w_out: Tensor) -> bool:
+def fused_mlp_ok(x: Tensor, w_in: Tensor, w_out: Tensor, reversed_: bool = False) -> bool:
+    if reversed_ and (w_in.size(1) % 8 or w_out.size(1) % 8):
+        return False
     return (x.is_cuda and x.dtype in _16BIT and w_in.dtype == x.dtype and w_out.dtype == x.dtype and x.numel() > 0
             and x.size(-1) % 8 == 0 and w_in.size(0) % 8 == 0 and w_out.size(0) % 8 == 0
             and x.numel() // x.size(-1) > SMALL_M_ROWS)
 
 
 def fused_mlp(x: Tensor, w_in: Tensor, b_in: Optional[Tensor], w_out: Tensor, b_out: Optional[Tensor],
-              residual: Optional[Tensor] = None) -> Tensor:
+              residual: Optional[Tensor] = None, reversed_: bool = False) -> Tensor:
     """``fc_out(gelu(fc_in(x))) (+ residual)``; the residual is added in fc_out's GEMM epilogue."""
-    return _FusedMLP.apply(x, w_in, b_in, w_out, b_out, residual)
+    return _FusedMLP.apply(x, w_in, b_in, w_out, b_out, residual, reversed_)
 
 
 class _QKVLinear(torch.autograd.Function):
@@ -560,6 +564,67 @@ def flash_attention(q: Tensor, k: Tensor, v: Tensor, causal: bool, window: Optio
 def decode_attention(q: Tensor, k_cache: Tensor, v_cache: Tensor, lengths: Tensor, scale: float,
                      window: Optional[int]) -> Tensor:
     return _ext().decode_attn(q.contiguous(), k_cache, v_cache, lengths.to(torch.int32), float(scale), int(window or 0))
+
+
+class _FlashPacked(torch.autograd.Function):
+    """Causal attention of ``qkv`` ``[B, S, 3 * heads * dim]`` (a projection's own output): the gradient is one tensor of that layout,
+    where the split's backward would join three."""
+
+    @staticmethod
+    def forward(ctx, qkv, heads, window, scale, kpm):
+        b, s, w3 = qkv.shape
+        q, k, v = qkv.view(b, s, 3, heads, w3 // 3 // heads).permute(2, 0, 3, 1, 4).unbind(0)
+        o, lse = _ext().flash_fwd(q, k, v, scale, True, window, kpm, _flash_impl())
+        ctx.save_for_backward(qkv, o, lse, kpm)
+        ctx.cfg = (heads, scale, window)
+        return o
+
+    @staticmethod
+    def backward(ctx, do):
+        qkv, o, lse, kpm = ctx.saved_tensors
+        heads, scale, window = ctx.cfg
+        b, s, w3 = qkv.shape
+        q, k, v = qkv.view(b, s, 3, heads, w3 // 3 // heads).permute(2, 0, 3, 1, 4).unbind(0)
+        dq, _, _ = _ext().flash_bwd(_attn_operand(do), q, k, v, o, lse, scale, True, window, kpm, _flash_impl())
+        return dq.as_strided((b, s, w3), (s * w3, w3, 1), dq.storage_offset()), None, None, None, None
+
+
+def packed_attention_ok(qkv: Tensor, heads: int) -> bool:
+    if not (qkv.is_cuda and qkv.dim() == 3 and qkv.is_contiguous() and qkv.data_ptr() % 16 == 0 and qkv.numel() > 0
+            and qkv.size(-1) % (24 * heads) == 0):
+        return False
+    q = qkv[..., :qkv.size(-1) // 3].unflatten(-1, (heads, -1)).permute(0, 2, 1, 3)
+    return flash_supported(q, q, q)
+
+
+def packed_attention(qkv: Tensor, heads: int, window: Optional[int], scale: float, key_padding_mask: Optional[Tensor]) -> Tensor:
+    """Causal attention ``[B, heads, S, dim]`` of a joint projection's output."""
+    kpm = (key_padding_mask != 0).to(torch.uint8).contiguous() if key_padding_mask is not None else None
+    return _FlashPacked.apply(qkv, heads, int(window or 0), float(scale), kpm)
+
+
+def prompt_append_ok(k: Tensor, v: Tensor, kc: Tensor, vc: Tensor) -> bool:
+    """Whether ``prompt_append`` copies ``k``, ``v`` ``[B, heads, S, D]`` into these caches."""
+    return (k.is_cuda and k.dtype in _16BIT and kc.dtype == k.dtype and v.dtype == k.dtype and vc.dtype == k.dtype
+            and k.shape == v.shape and kc.shape == vc.shape and k.numel() > 0 and k.size(-1) % 8 == 0
+            and kc.size(0) == k.size(0) and kc.size(1) == k.size(1) and kc.size(3) == k.size(3)
+            and kc.is_contiguous() and vc.is_contiguous() and kc.data_ptr() % 16 == 0 and vc.data_ptr() % 16 == 0
+            and all(t.stride(3) == 1 and t.data_ptr() % 16 == 0 and not any(s % 8 for s in t.stride()[:3]) for t in (k, v))
+            and not (torch.is_grad_enabled() and (k.requires_grad or v.requires_grad)))
+
+
+def prompt_append(k: Tensor, v: Tensor, kc: Tensor, vc: Tensor, start: int) -> None:
+    _ext().prompt_append(k, v, kc, vc, int(start))
+
+
+def rotary_own(x: Tensor, positions: Tensor, rotary_dim: int, base: float = 10000.0) -> Tensor:
+    """``rotary_interleaved`` of ``x`` ``[B, S, heads, D]``, a product's fresh output that nobody else holds, without gradients: in place."""
+    if not (x.is_contiguous() and x.size(3) % 8 == 0 and rotary_dim % 8 == 0 and x.data_ptr() % 16 == 0):
+        return rotary_interleaved(x, positions, rotary_dim, base)
+    if positions.dim() == 1:
+        positions = positions.unsqueeze(0).expand(x.size(0), -1)
+    _ext().rotary_(x, positions.to(torch.long).contiguous(), x.size(2), x.size(3), rotary_dim, base, False)
+    return x
 
 
 def decode_step_ok(q: Tensor, k_cache: Tensor, v_cache: Tensor) -> bool:

@@ -38,6 +38,10 @@ def register() -> None:
     def _(x1, x2, w, w_kn, bias, gelu_from, res=None, ln_w=None, ln_b=None, eps=0.0):
         return x1.new_empty((x1.size(0), (w[0].size(1) if w_kn else w[0].size(0)) * len(w)))
 
+    @reg("oslo_b200::prompt_append")
+    def _(k, v, kc, vc, start):
+        return None
+
     @reg("oslo_b200::decode_step_attn")
     def _(q, k, v, kc, vc, lengths, positions, write_index, rotary_dim, base, scale, window):
         return q.new_empty(q.shape)

@@ -63,8 +63,8 @@ class Conv1D(nn.Module):
     def out_features(self) -> int:
         return self.weight.size(1)
 
-    def forward(self, x: Tensor, activation: Optional[str] = None) -> Tensor:
-        return _linear(x, self.weight, self.bias, True, self.oslo_fused, activation)
+    def forward(self, x: Tensor, activation: Optional[str] = None, residual: Optional[Tensor] = None) -> Tensor:
+        return _linear(x, self.weight, self.bias, True, self.oslo_fused, activation, residual)
 
 
 class LayerNorm(nn.LayerNorm):

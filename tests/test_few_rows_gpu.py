@@ -77,3 +77,53 @@ def test_decode_step_attention(dtype, d, rotary, b, h, t, at, window):
     ref = torch.einsum("bht,bhtd->bhd", s.softmax(-1), v2[:, :, lo:at + 1].double())
     torch.testing.assert_close(out.double(), ref, atol=3 * EPS[dtype], rtol=3 * EPS[dtype])
     torch.testing.assert_close(cuda_ops.decode_attention(q, k2, v2, lengths, d ** -0.5, window or None).double(), ref, atol=3 * EPS[dtype], rtol=3 * EPS[dtype])
+
+
+@pytest.mark.parametrize("b, h, s, d, t, start", [(1, 1, 1, 8, 1, 0), (2, 3, 17, 64, 40, 5), (4, 16, 200, 256, 210, 10), (3, 5, 333, 80, 333, 0)])
+def test_prompt_append(b, h, s, d, t, start):
+    """Keys and values of a prompt land where slice copies put them, from slices of joint rows and from contiguous tensors."""
+    from oslo_b200.ops import cuda_ops
+    for k, v in (torch.randn(b, s, 2, h, d, device="cuda").bfloat16().permute(2, 0, 3, 1, 4).unbind(0),
+                 (torch.randn(b, h, s, d, device="cuda").bfloat16(), torch.randn(b, s, h, d, device="cuda").bfloat16().transpose(1, 2))):
+        kc, vc = (torch.randn(b, h, t, d, device="cuda").bfloat16() for _ in range(2))
+        k2, v2 = kc.clone(), vc.clone()
+        assert cuda_ops.prompt_append_ok(k, v, k2, v2)
+        cuda_ops.prompt_append(k, v, k2, v2, start)
+        kc[:, :, start:start + s], vc[:, :, start:start + s] = k, v
+        assert torch.equal(k2, kc) and torch.equal(v2, vc)
+
+
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("b, s, h, d, window", [(2, 65, 3, 64, 0), (1, 300, 2, 128, 40)])
+def test_packed_attention_is_the_split_one(b, s, h, d, window, masked):
+    from oslo_b200.ops import cuda_ops
+    torch.manual_seed(s)
+    qkv = torch.randn(b, s, 3 * h * d, device="cuda").bfloat16().requires_grad_()
+    mask = (torch.arange(s, device="cuda") < s - 7).long().expand(b, s) if masked else None
+    g = torch.randn(b, h, s, d, device="cuda").bfloat16()
+    a = cuda_ops.packed_attention(qkv, h, window or None, d ** -0.5, mask)
+    ga, = torch.autograd.grad(a, qkv, g)
+    q, k, v = (x.unflatten(-1, (h, d)).transpose(1, 2) for x in qkv.split(h * d, dim=2))
+    c = cuda_ops.flash_attention(q, k, v, True, window or None, d ** -0.5, mask)
+    gc, = torch.autograd.grad(c, qkv, g)
+    assert torch.equal(a, c) and torch.equal(ga, gc)
+
+
+@pytest.mark.parametrize("reversed_", [False, True])
+def test_fused_mlp_layouts(reversed_):
+    """Both weight layouts of the two-layer node against 64-bit autograd: one rounding of each of four 16-bit intermediates."""
+    from oslo_b200.ops import cuda_ops
+    torch.manual_seed(1)
+    n, w, f = 200, 72, 264
+    p = [torch.randn(*s, device="cuda") * sc for s, sc in (((n, w), 1), ((f, w), 0.1), ((f,), 0.1), ((w, f), 0.1), ((w,), 0.1), ((n, w), 1))]
+    p = [x.bfloat16().requires_grad_() for x in p]
+    x, w1, b1, w2, b2, r = p
+    g = torch.randn(n, w, device="cuda").bfloat16()
+    a, c = (w1.t().contiguous(), w2.t().contiguous()) if reversed_ else (w1, w2)
+    y = cuda_ops.fused_mlp(x, a, b1, c, b2, r, reversed_)
+    got = torch.autograd.grad(y, p, g)
+    d = [t.detach().double().requires_grad_() for t in p]
+    ref = torch.nn.functional.gelu(d[0] @ d[1].t() + d[2], approximate="tanh") @ d[3].t() + d[4] + d[5]
+    want = torch.autograd.grad(ref, d, g.double())
+    for have, need in zip((y, *got), (ref, *want)):
+        assert (have.double() - need).norm() <= 4 * 2.0 ** -8 * need.norm()
