@@ -50,6 +50,10 @@ struct GemmParams {
   int* err;
   int tiles_m, tiles_n;
   int group_m = 8;      // row blocks per column sweep of the tile raster
+  // CTA pairs: the tiles from split_from on are cut into `split` ranges of k whose fp32 sums go to split_ws
+  // [tiles - split_from][split][256][256]; split_finish_kernel adds them up and runs the epilogue
+  int split = 1, split_from = 0;
+  float* split_ws = nullptr;
   // cross-entropy epilogues (GEMM_FLAG_CE_STATS / GEMM_FLAG_CE_GRAD)
   const long long* ce_labels = nullptr;   // [M] global vocabulary ids
   long long ce_vocab_start = 0;           // id of this matrix's column 0

@@ -67,8 +67,17 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  const int num_tiles = p.tiles_m * p.tiles_n;    // 256 x 256 tiles
+  // work items: whole tiles, then the ranges of k of the last ones (range ks of all of them before range ks + 1)
   const int kblocks = (p.K + BK - 1) / BK;
+  const int whole = p.split > 1 ? p.split_from : p.tiles_m * p.tiles_n, cut = p.tiles_m * p.tiles_n - whole;
+  const int items = whole + cut * p.split;
+  auto unpack = [&](int item, int& tile, int& ks, int& kb0, int& kb1) {
+    const int j = item - whole;
+    ks = j < 0 ? 0 : j / cut;
+    tile = j < 0 ? item : whole + j % cut;
+    kb0 = j < 0 ? 0 : ks * kblocks / p.split;
+    kb1 = j < 0 ? kblocks : (ks + 1) * kblocks / p.split;
+  };
   const int cluster_id = blockIdx.x >> 1;
   const int n_clusters = gridDim.x >> 1;
 
@@ -80,12 +89,13 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int tile = cluster_id; tile < num_tiles && ok; tile += n_clusters) {
-        int tm, tn;
+      for (int item = cluster_id; item < items && ok; item += n_clusters) {
+        int tile, ks, kb0, kb1, tm, tn;
+        unpack(item, tile, ks, kb0, kb1);
         tile_coords(tile, p.tiles_m, p.tiles_n, tm, tn, p.group_m);
         const int m0 = tm * PAIR_TILE + static_cast<int>(rank) * BM;
         const int n0 = tn * PAIR_TILE + static_cast<int>(rank) * BM;
-        for (int kb = 0; kb < kblocks; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           ok = mbar_wait(empty_bar(stage), phase ^ 1, abort_flag, p.err, ERR_WAIT_EMPTY);
           if (!ok) break;
           const uint32_t sa = smem_base + stage * STAGE_BYTES;
@@ -123,14 +133,16 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
       uint32_t acc_phase[2] = {0, 0};
       int local = 0;
       bool ok = true;
-      for (int tile = cluster_id; tile < num_tiles && ok; tile += n_clusters, ++local) {
+      for (int item = cluster_id; item < items && ok; item += n_clusters, ++local) {
+        int tile, ks, kb0, kb1;
+        unpack(item, tile, ks, kb0, kb1);
         const int buf = local & 1;
         ok = mbar_wait(tempty_bar(buf), acc_phase[buf] ^ 1, abort_flag, p.err, ERR_WAIT_TMEM_EMPTY);
         if (!ok) break;
         acc_phase[buf] ^= 1;
         tc_fence_after();
         const uint32_t tmem_acc = tmem_base + buf * PAIR_TILE;
-        for (int kb = 0; kb < kblocks; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           ok = mbar_wait(full_bar(stage), phase, abort_flag, p.err, ERR_WAIT_FULL);
           if (!ok) break;
           tc_fence_after();
@@ -140,7 +152,7 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
           for (int k = 0; k < BK / 16; ++k) {
             const uint64_t da = make_smem_desc(sa + k * a_step, a_lbo, 1024);
             const uint64_t db = make_smem_desc(sb + k * b_step, b_lbo, 1024);
-            umma_f16_pair(tmem_acc, da, db, idesc, (kb | k) != 0);
+            umma_f16_pair(tmem_acc, da, db, idesc, kb != kb0 || k != 0);
           }
           umma_commit_pair(empty_bar(stage));                  // this CTA's stage ...
           umma_commit_pair(map_to_cta(empty_bar(stage), 1));   // ... and the peer's
@@ -160,9 +172,10 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
     uint32_t acc_phase[2] = {0, 0};
     int local = 0;
     bool ok = true;
-    for (int tile = cluster_id; tile < num_tiles && ok; tile += n_clusters, ++local) {
+    for (int item = cluster_id; item < items && ok; item += n_clusters, ++local) {
       const int buf = local & 1;
-      int tm, tn;
+      int tile, ks, kb0, kb1, tm, tn;
+      unpack(item, tile, ks, kb0, kb1);
       tile_coords(tile, p.tiles_m, p.tiles_n, tm, tn, p.group_m);
       ok = mbar_wait_warp(tfull_bar(buf), acc_phase[buf], abort_flag, p.err, ERR_WAIT_TMEM_FULL);
       if (!ok) break;
@@ -182,7 +195,13 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
         tmem_wait_ld();
         const int col0 = tn * PAIR_TILE + c0;
         if (!row_ok || col0 >= p.N) continue;
-        if (ce_stats) {
+        if (item >= whole) {
+          float4* w = reinterpret_cast<float4*>(p.split_ws + (static_cast<size_t>(tile - whole) * p.split + ks) * (PAIR_TILE * PAIR_TILE) +
+                                                (static_cast<int>(rank) * BM + quad * 32 + lane) * PAIR_TILE + c0);
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            w[i] = make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]), __uint_as_float(r[4 * i + 2]), __uint_as_float(r[4 * i + 3]));
+        } else if (ce_stats) {
           ce_accumulate(p, col0, r, fp16, label_local, ce);
           ce_flush_if_block_ends(p, row, col0, ce);
         } else {
@@ -206,6 +225,40 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
     tc_fence_after();
     tmem_dealloc_pair(tmem_base, TMEM_COLS);
   }
+}
+
+// The sums of the ranges of k, in their order, and the epilogue, for FINISH_ROWS rows of a cut tile: whole rows of every range are on
+// their way together (a thread that read its 32 columns range by range took 10 us for two tiles of eight ranges), then one thread
+// per row and 32 columns runs the epilogue.
+constexpr int FINISH_ROWS = 8, FINISH_SPLIT = 8;
+__global__ void __launch_bounds__(256) split_finish_kernel(const GemmParams p) {
+  __shared__ __align__(16) float sum[FINISH_ROWS][PAIR_TILE + 4];
+  const int j = blockIdx.x / (PAIR_TILE / FINISH_ROWS), row0 = (blockIdx.x % (PAIR_TILE / FINISH_ROWS)) * FINISH_ROWS;
+  int tm, tn;
+  tile_coords(p.split_from + j, p.tiles_m, p.tiles_n, tm, tn, p.group_m);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const float4* w = reinterpret_cast<const float4*>(p.split_ws + static_cast<size_t>(j) * p.split * (PAIR_TILE * PAIR_TILE) + row0 * PAIR_TILE);
+#pragma unroll
+  for (int u = 0; u < FINISH_ROWS * PAIR_TILE / 4 / 256; ++u) {
+    const int e = u * 256 + threadIdx.x, r = e / (PAIR_TILE / 4), c = (e % (PAIR_TILE / 4)) * 4;
+    if (tm * PAIR_TILE + row0 + r >= p.M || tn * PAIR_TILE + c / 32 * 32 >= p.N) continue;   // never written
+    float4 q[FINISH_SPLIT];
+#pragma unroll
+    for (int s = 0; s < FINISH_SPLIT; ++s) q[s] = s < p.split ? w[s * (PAIR_TILE * PAIR_TILE / 4) + e] : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 v = q[0];
+#pragma unroll
+    for (int s = 1; s < FINISH_SPLIT; ++s) { v.x += q[s].x; v.y += q[s].y; v.z += q[s].z; v.w += q[s].w; }
+    *reinterpret_cast<float4*>(&sum[r][c]) = v;
+  }
+  __syncthreads();
+  if (threadIdx.x >= FINISH_ROWS * (PAIR_TILE / 32)) return;
+  const int r = threadIdx.x / (PAIR_TILE / 32), c0 = (threadIdx.x % (PAIR_TILE / 32)) * 32;
+  const int row = tm * PAIR_TILE + row0 + r, col0 = tn * PAIR_TILE + c0;
+  if (row >= p.M || col0 >= p.N) return;
+  uint32_t v[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(sum[r][c0 + i]);
+  epilogue_chunk(p, row, col0, v, (p.flags & GEMM_FLAG_FP16) != 0, (p.flags & GEMM_FLAG_OUT_FP32) != 0);
 }
 
 }  // namespace oslo

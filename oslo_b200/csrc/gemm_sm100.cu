@@ -110,7 +110,7 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams&
   p.tiles_n = (p.N + PAIR_TILE - 1) / PAIR_TILE;
   static const int group_m = [] { const char* e = getenv("OSLO_B200_GEMM_GROUP_M"); const int v = e ? atoi(e) : 8; return v > 0 ? v : 8; }();
   p.group_m = group_m;
-  const int tiles = p.tiles_m * p.tiles_n;
+  const int tiles = p.split > 1 ? p.split_from + (p.tiles_m * p.tiles_n - p.split_from) * p.split : p.tiles_m * p.tiles_n;
   // persistent kernel: no more pairs than can be resident at once (pairs are placed as clusters of two SMs)
   static int max_pairs = 0;
   if (max_pairs == 0) {
@@ -124,7 +124,17 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams&
   }
   const int pairs = std::min(tiles, std::min(max_pairs, num_sms / 2));   // num_sms already excludes reserved SMs
   gemm_pair_tcgen05_kernel<STAGES><<<2 * pairs, GEMM_THREADS, smem, stream>>>(ta, tb, p);
-  return static_cast<int>(cudaGetLastError());
+  if (p.split <= 1) return static_cast<int>(cudaGetLastError());
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3(static_cast<unsigned>((p.tiles_m * p.tiles_n - p.split_from) * (PAIR_TILE / FINISH_ROWS)));
+  cfg.blockDim = dim3(256);
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, split_finish_kernel, static_cast<const GemmParams>(p)));
 }
 
 // 0 = single-CTA tiles only (OSLO_B200_GEMM_PAIR=0), 1 = CTA pairs for large outputs (default)
@@ -133,15 +143,43 @@ static bool pair_enabled() {
   return on;
 }
 
+// Into how many ranges of k the tiles of a pair GEMM's last, incomplete wave are cut (1: none). With R tiles on P pairs, ranges of 1/s
+// of k take ceil(R s / P) / s of a wave. A k block of a wave takes about 0.4 us; the second
+// kernel and the ranges' own pipeline fills cost about 8 us and a range 0.1 us for its 256 KB there and back. bf16, uncut and cut:
+// 3062 x 2048, k = 8192: 94.5 and 83.7 us; 7108 x 2048, k = 8192: 251 and 215; 768 x 768, k = 8000: 57.8 and 29.1; 4096 x 768,
+// k = 50264: 291 and 240; where the rule says no, 7108 x 2048, k = 2048: 80.3 and 82.3 (cut in four).
+static int pair_split(int M, int N, int K, int num_sms) {
+  const int P = num_sms / 2, kblocks = (K + BK - 1) / BK;
+  const long long tiles = static_cast<long long>((M + PAIR_TILE - 1) / PAIR_TILE) * ((N + PAIR_TILE - 1) / PAIR_TILE);
+  const int R = static_cast<int>(tiles % P);
+  if (R == 0) return 1;
+  int best = 1;
+  double most = 2.0;                            // what it has to give at least, us
+  for (int s = 2; s <= FINISH_SPLIT && kblocks >= 8 * s && R * s <= 2 * P; ++s) {
+    const double gain = (1.0 - static_cast<double>((R * s + P - 1) / P) / s) * kblocks * 0.4 - 8.0 - 0.1 * R * s;
+    if (gain > most) { most = gain; best = s; }
+  }
+  return best;
+}
+
 // Tile shape selection, tensor maps and launch for a filled-in GemmParams (M, N, K, majors, flags, epilogue operands)
 static int dispatch_gemm(const void* A, const void* B, int lda, int ldb, GemmParams& p, int num_sms, cudaStream_t stream);
 
 }  // namespace oslo
 
+// floats of workspace with which oslo_gemm_16bit cuts the last wave's tiles (0: it does not)
+extern "C" long long oslo_gemm_split_floats(int M, int N, int K, int num_sms) {
+  using namespace oslo;
+  if (!pair_enabled() || M < PAIR_TILE || N < PAIR_TILE || K <= 0) return 0;
+  const int s = pair_split(M, N, K, num_sms);
+  const long long tiles = static_cast<long long>((M + PAIR_TILE - 1) / PAIR_TILE) * ((N + PAIR_TILE - 1) / PAIR_TILE);
+  return s > 1 ? tiles % (num_sms / 2) * s * PAIR_TILE * PAIR_TILE : 0;
+}
+
 extern "C" int oslo_gemm_16bit(const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb, int ldd,
                                int a_mn_major, int b_mn_major, const void* bias, const void* aux, int ld_aux,
-                               void* aux_out, int ld_aux_out, int flags, float alpha, int* err_word, int num_sms,
-                               cudaStream_t stream) {
+                               void* aux_out, int ld_aux_out, int flags, float alpha, float* split_ws, int* err_word,
+                               int num_sms, cudaStream_t stream) {
   using namespace oslo;
   if (M <= 0 || N <= 0 || K <= 0) return -1;
   if (flags & (GEMM_FLAG_CE_STATS | GEMM_FLAG_CE_GRAD | GEMM_FLAG_GLU)) return -7;   // those epilogues come through oslo_gemm_ce_16bit
@@ -149,6 +187,7 @@ extern "C" int oslo_gemm_16bit(const void* A, const void* B, void* D, int M, int
   p.D = D; p.bias = bias; p.aux = aux; p.aux_out = aux_out;
   p.M = M; p.N = N; p.K = K; p.ldd = ldd; p.ld_aux = ld_aux; p.ld_aux_out = ld_aux_out;
   p.a_mn_major = a_mn_major; p.b_mn_major = b_mn_major; p.flags = flags; p.alpha = alpha; p.err = err_word;
+  p.split_ws = split_ws;
   p.comm = CommParams{};
   return dispatch_gemm(A, B, lda, ldb, p, num_sms, stream);
 }
@@ -180,9 +219,16 @@ static int dispatch_gemm(const void* A, const void* B, int lda, int ldb, GemmPar
   const bool fp16 = (flags & GEMM_FLAG_FP16) != 0;
   // narrow outputs use the 128-wide tile so that more CTAs share the work
   const bool wide = (N >= 256) && (static_cast<long long>((M + BM - 1) / BM) * ((N + 255) / 256) >= num_sms / 2);
-  // large outputs: 256 x 256 tiles on CTA pairs, when they fill the pairs at least as well as single tiles fill the SMs
+  // large outputs: 256 x 256 tiles on CTA pairs. They pull a third to a half less operand data out of L2 per FLOP and win with half of
+  // the pairs idle (bf16, k = 7108, 2048 x 2048, 64 tiles: 55.8 us, 63.4 on 128 x 256 and 90.4 on 128 x 128 tiles; k = 50264,
+  // 4096 x 768, 48 tiles: 264, 298, 461), not with more (k = 8000, 768 x 3072, 36 tiles: 53.9, 60.0, 49.5), except where the idle ones
+  // take ranges of k
   const long long pair_tiles = static_cast<long long>((M + PAIR_TILE - 1) / PAIR_TILE) * ((N + PAIR_TILE - 1) / PAIR_TILE);
-  const bool pair = pair_enabled() && wide && M >= PAIR_TILE && pair_tiles >= num_sms / 2;
+  if (p.split_ws != nullptr) {
+    p.split = pair_split(M, N, K, num_sms);
+    p.split_from = static_cast<int>(pair_tiles - pair_tiles % (num_sms / 2));
+  }
+  const bool pair = pair_enabled() && M >= PAIR_TILE && N >= PAIR_TILE && (pair_tiles >= num_sms / 4 + 1 || p.split > 1);
   const int bn = pair ? BM : (wide ? 256 : 128);   // B box rows: a pair's CTA stages 128 of the 256 tile columns
   CUtensorMap ta, tb;
   int rc;

@@ -64,3 +64,29 @@ def test_layernorm_rows_at_the_edges_of_its_layouts(rows, cols, dtype):
     assert _rel(y, want) < 2 * unit
     for leaf, ref in zip(leaves, wide):
         assert _rel(leaf.grad, ref.grad) < 2 * unit, leaf.shape
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("a_mn, b_mn", [(False, False), (False, True), (True, True)])
+@pytest.mark.parametrize("m, n, k", [(768, 768, 8000), (300, 264, 4104), (768, 2304, 8008), (3062, 2048, 8192), (257, 8192, 6000)])
+def test_gemm_tiles_cut_along_k(m, n, k, a_mn, b_mn, dtype):
+    """The last wave's tiles as ranges of k: every epilogue that they can meet, against 64 bits; the sums stay 32 bits wide."""
+    from oslo_b200.ops import cuda_ops as co
+    torch.manual_seed(m + n)
+    m8 = m if not a_mn else -(-m // 8) * 8
+    a = torch.randn(*((k, m8) if a_mn else (m8, k)), device="cuda").to(dtype)
+    b = (torch.randn(*((k, n) if b_mn else (n, k)), device="cuda") * k ** -0.5).to(dtype)
+    bias, aux = torch.randn(n, device="cuda").to(dtype), torch.randn(m8, n, device="cuda").to(dtype)
+    z = (a.double().t() if a_mn else a.double()) @ (b.double() if b_mn else b.double().t())
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    out = aux.clone()
+    pre = torch.empty_like(aux)
+    g = torch.nn.functional.gelu
+    for got, want in ((co.gemm(a, b, a_mn, b_mn), z),
+                      (co.gemm(a, b, a_mn, b_mn, bias=bias, aux=aux, flags=co.FLAG_BIAS | co.FLAG_RESIDUAL), z + bias.double() + aux.double()),
+                      (co.gemm(a, b, a_mn, b_mn, out=out, flags=co.FLAG_ACCUMULATE), z + aux.double()),
+                      (co.gemm(a, b, a_mn, b_mn, bias=bias, aux_out=pre, flags=co.FLAG_BIAS | co.FLAG_GELU | co.FLAG_SAVE_PREACT),
+                       g(z + bias.double(), approximate="tanh")), (pre, z + bias.double())):
+        assert _rel(got, want) <= eps             # one rounding; GeLU's tanh is good to 2^-11
+    y = co.gemm(a, b, a_mn, b_mn, flags=co.FLAG_OUT_FP32)
+    assert _rel(y, z) <= 1e-5                     # 32-bit sums of k products: sqrt(8192) roundings of 2^-24, twice over
