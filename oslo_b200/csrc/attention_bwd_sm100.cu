@@ -41,38 +41,40 @@ struct FaBwdParams {
   int* err;
 };
 
-// delta[b, h, q] = sum_d dO[b, h, q, d] * O[b, h, q, d]; one warp per row
-template <typename T>
-__global__ void fa_delta_kernel(const T* __restrict__ o, const T* __restrict__ dout, float* __restrict__ delta, int B,
-                                int H, int Sq, int D, long long o_sb, long long o_sh, long long o_ss, long long d_sb,
-                                long long d_sh, long long d_ss) {
-  const long long row = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= static_cast<long long>(B) * H * Sq) return;
-  const int q = static_cast<int>(row % Sq);
-  const int h = static_cast<int>((row / Sq) % H);
-  const int b = static_cast<int>(row / (static_cast<long long>(Sq) * H));
-  const T* op = o + b * o_sb + h * o_sh + q * o_ss;
-  const T* dp = dout + b * d_sb + h * d_sh + q * d_ss;
+// delta[b, h, q] = sum_d dO[b, h, q, d] * O[b, h, q, d]; D / 8 lanes per row, 16 bytes each, rows in the order (b, q, h) in which a
+// projection's gradient lies in memory. Bound by reading both: 8 x 12 x 1000 x 64: 24 us with a warp and 4 bytes a lane per row.
+template <typename T> __device__ __forceinline__ float delta_dot(const uint4& a, const uint4& g) {
+  const uint32_t x[4] = {a.x, a.y, a.z, a.w}, y[4] = {g.x, g.y, g.z, g.w};
   float acc = 0.f;
-  for (int d = lane * 2; d < D; d += 64) {
-    const uint32_t a = *reinterpret_cast<const uint32_t*>(op + d);
-    const uint32_t g = *reinterpret_cast<const uint32_t*>(dp + d);
-    float a0, a1, g0, g1;
-    if (sizeof(T) == 2 && std::is_same<T, __half>::value) {
-      const float2 fa = __half22float2(*reinterpret_cast<const __half2*>(&a));
-      const float2 fg = __half22float2(*reinterpret_cast<const __half2*>(&g));
-      a0 = fa.x; a1 = fa.y; g0 = fg.x; g1 = fg.y;
-    } else {
-      const float2 fa = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a));
-      const float2 fg = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g));
-      a0 = fa.x; a1 = fa.y; g0 = fg.x; g1 = fg.y;
-    }
-    acc += a0 * g0 + a1 * g1;
-  }
 #pragma unroll
-  for (int s = 16; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
-  if (lane == 0) delta[row] = acc;
+  for (int i = 0; i < 4; ++i) {
+    float2 p, q;
+    if constexpr (std::is_same<T, __half>::value) {
+      p = __half22float2(*reinterpret_cast<const __half2*>(&x[i]));
+      q = __half22float2(*reinterpret_cast<const __half2*>(&y[i]));
+    } else {
+      p = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x[i]));
+      q = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&y[i]));
+    }
+    acc += p.x * q.x + p.y * q.y;
+  }
+  return acc;
+}
+template <typename T, int D>
+__global__ void __launch_bounds__(256) fa_delta_kernel(const T* __restrict__ o, const T* __restrict__ dout, float* __restrict__ delta, int B,
+                                                       int H, int Sq, long long o_sb, long long o_sh, long long o_ss, long long d_sb,
+                                                       long long d_sh, long long d_ss) {
+  constexpr int LPR = D / 8, ROWS = 256 / LPR;
+  const long long row = static_cast<long long>(blockIdx.x) * ROWS + threadIdx.x / LPR, rows = static_cast<long long>(B) * H * Sq;
+  const int d = (threadIdx.x % LPR) * 8;
+  const bool in = row < rows;
+  const long long r = in ? row : 0;
+  const int h = static_cast<int>(r % H), q = static_cast<int>((r / H) % Sq), b = static_cast<int>(r / (static_cast<long long>(H) * Sq));
+  float acc = delta_dot<T>(*reinterpret_cast<const uint4*>(o + b * o_sb + h * o_sh + q * o_ss + d),
+                           *reinterpret_cast<const uint4*>(dout + b * d_sb + h * d_sh + q * d_ss + d));
+#pragma unroll
+  for (int s = LPR / 2; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+  if (in && d == 0) delta[(static_cast<long long>(b) * H + h) * Sq + q] = acc;
 }
 
 __device__ __forceinline__ bool fa_visible(int q, int k, int offset, int Sq, int Sk, int causal, int window) {
@@ -476,15 +478,20 @@ extern "C" int oslo_flash_bwd_sm100(const void* q, const void* k, const void* v,
   const bool fp16 = dtype == OSLO_DT_FP16;
   {
     const long long rows = static_cast<long long>(B) * H * Sq;
-    const int wpb = 8;
-    const unsigned blocks = static_cast<unsigned>((rows + wpb - 1) / wpb);
-    if (fp16)
-      fa_delta_kernel<__half><<<blocks, wpb * 32, 0, stream>>>(static_cast<const __half*>(o), static_cast<const __half*>(dout),
-                                                               delta, B, H, Sq, D, o_sb, o_sh, o_ss, do_sb, do_sh, do_ss);
-    else
-      fa_delta_kernel<__nv_bfloat16><<<blocks, wpb * 32, 0, stream>>>(static_cast<const __nv_bfloat16*>(o),
-                                                                      static_cast<const __nv_bfloat16*>(dout), delta, B, H,
-                                                                      Sq, D, o_sb, o_sh, o_ss, do_sb, do_sh, do_ss);
+    const int per = 256 / (D / 8);
+    const unsigned blocks = static_cast<unsigned>((rows + per - 1) / per);
+#define FA_DELTA(T, DD) fa_delta_kernel<T, DD><<<blocks, 256, 0, stream>>>(static_cast<const T*>(o), static_cast<const T*>(dout), delta, B, H, Sq, \
+                                                                          o_sb, o_sh, o_ss, do_sb, do_sh, do_ss)
+#define FA_DELTA_T(T)                   \
+  do {                                  \
+    if (D == 64) FA_DELTA(T, 64);       \
+    else if (D == 128) FA_DELTA(T, 128);\
+    else FA_DELTA(T, 256);              \
+  } while (0)
+    if (fp16) FA_DELTA_T(__half);
+    else FA_DELTA_T(__nv_bfloat16);
+#undef FA_DELTA_T
+#undef FA_DELTA
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return static_cast<int>(e);
   }

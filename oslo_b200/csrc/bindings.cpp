@@ -265,6 +265,17 @@ Tensor gemm_small_m(const Tensor& a, const Tensor& b, int64_t b_mn, const option
   return few_rows(a, optional<Tensor>(), {b}, b_mn, bias, gelu_from, optional<Tensor>(), optional<Tensor>(), optional<Tensor>(), 0.0);
 }
 
+// grad [V, W] += rows of dy [n, W] by ids [n]
+void embedding_grad_(Tensor grad, const Tensor& ids, const Tensor& dy) {
+  TORCH_CHECK(grad.is_cuda() && grad.dim() == 2 && grad.is_contiguous() && dy.dim() == 2 && dy.is_contiguous() && dy.size(1) == grad.size(1) &&
+                  dy.scalar_type() == grad.scalar_type() && dy.device() == grad.device(), "embedding_grad: grad and dy");
+  TORCH_CHECK(ids.scalar_type() == at::kLong && ids.is_contiguous() && ids.numel() == dy.size(0) && ids.device() == grad.device(), "embedding_grad: ids");
+  c10::cuda::CUDAGuard guard(grad.device());
+  check_rc(oslo_embedding_grad(reinterpret_cast<const long long*>(ids.data_ptr<int64_t>()), dy.data_ptr(), grad.data_ptr(),
+                               static_cast<int>(dy.size(0)), grad.size(0), static_cast<int>(grad.size(1)), dt_code(grad),
+                               dev_state(grad.get_device()).err.data_ptr<int>(), cur_stream()), "embedding_grad");
+}
+
 std::tuple<Tensor, Tensor, Tensor> layernorm_fwd(const Tensor& x, const Tensor& w, const optional<Tensor>& b, double eps) {
   TORCH_CHECK(x.is_cuda() && x.is_contiguous() && w.is_contiguous(), "layernorm: contiguous CUDA tensors required");
   c10::cuda::CUDAGuard guard(x.device());
@@ -1820,6 +1831,7 @@ TORCH_LIBRARY(oslo_b200, m) {
   m.def("flash_bwd(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse, float scale, bool causal, int window, Tensor? kpm, int impl=1) -> (Tensor, Tensor, Tensor)");
   m.def("decode_attn(Tensor q, Tensor kc, Tensor vc, Tensor lengths, float scale, int window) -> Tensor");
   m.def("gemm_comm(Tensor a, Tensor b, int a_mn, int b_mn, Tensor? bias, Tensor? aux, Tensor(a!)? aux_out, Tensor(b!)? out, int flags, float alpha, int M, int N, int K, int peer_bufs_dev, int own_buf, int mc_base, int data_off, int flag_off, int flag_bytes, int rank, int world, int epoch, int done_base, int mode, bool use_multimem, Tensor(c!)? trace) -> int");
+  m.def("embedding_grad_(Tensor(a!) grad, Tensor ids, Tensor dy) -> ()");
   m.def("few_rows(Tensor x1, Tensor? x2, Tensor[] w, int w_kn, Tensor? bias, int gelu_from, Tensor? res=None, Tensor? ln_w=None, "
         "Tensor? ln_b=None, float eps=0.0) -> Tensor");
   m.def("prompt_append(Tensor k, Tensor v, Tensor(a!) kc, Tensor(b!) vc, int start) -> ()");
@@ -1899,6 +1911,7 @@ TORCH_LIBRARY_IMPL(oslo_b200, CUDA, m) {
   m.impl("flash_bwd", &flash_bwd);
   m.impl("decode_attn", &decode_attn);
   m.impl("gemm_comm", &gemm_comm);
+  m.impl("embedding_grad_", &embedding_grad_);
   m.impl("few_rows", &few_rows);
   m.impl("prompt_append", &prompt_append);
   m.impl("decode_step_attn", &decode_step_attn);

@@ -47,6 +47,12 @@ int oslo_gemm_ce_16bit(const void* A, const void* B, int M, int N, int K, int ld
 int oslo_ce_reduce_stats(const float* stats, float* rowmax, float* sumexp, float* target, int rows, int blocks,
                          cudaStream_t stream);
 
+// grad [vocab, width] (16-bit) += rows of dy [n, width] by id; n <= OSLO_EMBED_GRAD_TOKENS, width % 8 == 0; ids outside the vocabulary
+// are skipped
+#define OSLO_EMBED_GRAD_TOKENS 32768
+int oslo_embedding_grad(const long long* ids, const void* dy, void* grad, int n, long long vocab, int width, int dtype, int* err_word,
+                        cudaStream_t stream);
+
 // LayerNorm over the last dim of [rows, cols]; mean/rstd are fp32 [rows]
 int oslo_layernorm_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd, int rows,
                        int cols, float eps, int dtype, cudaStream_t stream);

@@ -313,6 +313,89 @@ __global__ void __launch_bounds__(THREADS) branch_join_kernel(const BranchParams
   }
 }
 
+// The same for many rows of 16-bit branches without a convolution: a thread holds K chunks of eight columns of the whole row, all loads
+// of the row are on their way before the first is used, and nothing is read again (above, a branch with a norm is read twice, the row
+// goes through shared memory, and the loads of a chunk wait for the chunk before).
+template <typename T, int K>
+__global__ void __launch_bounds__(256, K == 1 ? 3 : 2) branch_join_rows_kernel(const BranchParams p) {
+  __shared__ float red[32];
+  const long long row = blockIdx.x;
+  const int step = blockDim.x * 8, c0 = threadIdx.x * 8;
+  float v[K][8], y[3][K][8];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int c = c0 + k * step;
+    const bool in = c < p.cols;
+    if (in) load_vec<float, 4>(p.x + row * p.cols + c, reinterpret_cast<float (&)[4]>(v[k][0]));
+    if (in) load_vec<float, 4>(p.x + row * p.cols + c + 4, reinterpret_cast<float (&)[4]>(v[k][4]));
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
+      if (b < p.n && in) load_branch<T, 8>(p, b, row, c, y[b][k]);
+    if (!in) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[k][i] = y[0][k][i] = y[1][k][i] = y[2][k][i] = 0.f;
+    }
+  }
+#pragma unroll
+  for (int b = 0; b < 3; ++b) {
+    if (b >= p.n) break;
+    float f = p.mult * p.factor[b];
+    if (p.w[b] != nullptr && p.normed[b]) {                // uniform over the block
+      float ss = 0.f;
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) ss = fmaf(y[b][k][i], y[b][k][i], ss);
+      ss = block_sum(ss, red);
+      f *= 1.0f / sqrtf(ss / p.cols + p.eps);
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int c = c0 + k * step;
+      if (c >= p.cols) continue;
+      if (p.w[b] != nullptr) {
+        float w[8];
+        load_vec<T, 8>(static_cast<const T*>(p.w[b]) + c, w);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[k][i] = fmaf(f * y[b][k][i], w[i], v[k][i]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[k][i] = fmaf(f, y[b][k][i], v[k][i]);
+      }
+    }
+  }
+  float sx = 0.f;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int c = c0 + k * step;
+    if (c >= p.cols) continue;
+    store_vec<float, 4>(p.x_out + row * p.cols + c, reinterpret_cast<const float (&)[4]>(v[k][0]));
+    store_vec<float, 4>(p.x_out + row * p.cols + c + 4, reinterpret_cast<const float (&)[4]>(v[k][4]));
+    if (p.copy) store_vec<T, 8>(static_cast<T*>(p.h1) + row * p.cols + c, v[k]);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) sx = fmaf(v[k][i], v[k][i], sx);
+  }
+  if (p.w1 == nullptr) return;
+  sx = block_sum(sx, red);
+  const float rn = 1.0f / sqrtf(sx / p.cols + p.eps);
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int c = c0 + k * step;
+    if (c >= p.cols) continue;
+    float w[8], h[8];
+    load_weight<T, 8>(p.w1, p.one1, c, w);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) h[i] = v[k][i] * rn * w[i];
+    store_vec<T, 8>(static_cast<T*>(p.h1) + row * p.cols + c, h);
+    if (p.w2 != nullptr) {
+      load_weight<T, 8>(p.w2, p.one2, c, w);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) h[i] = v[k][i] * rn * w[i];
+      store_vec<T, 8>(static_cast<T*>(p.h2) + row * p.cols + c, h);
+    }
+  }
+}
+
 // out[r, c] = gelu_tanh(z[r, c]) * table[ids[r], first + c]; a token outside the table counts as one with zeros
 template <typename T, int VEC>
 __global__ void __launch_bounds__(256) token_gate_kernel(const T* __restrict__ z, long long ldz, const long long* __restrict__ ids,
@@ -526,6 +609,19 @@ extern "C" int oslo_branch_join(const OsloBranchJoin* a, long long rows, int col
   if (smem > 200 * 1024) return -3;
   const int threads = cols >= 1024 ? 256 : (cols >= 512 ? 128 : 64);
   const bool few = rows <= 296 && cols > 1024;         // at most two blocks per SM
+  bool wide = !few && te == 2 && vec && cols % 8 == 0 && cols >= 512 && cols <= 4096 && a->conv_w == nullptr && rows > 296;
+  for (const void* t : {static_cast<const void*>(a->h1), static_cast<const void*>(a->h2), a->one1 ? nullptr : a->w1, a->one2 ? nullptr : a->w2})
+    wide = wide && aligned_to(t, 16);
+  for (int i = 0; i < p.n; ++i) wide = wide && p.ldy[i] % 8 == 0 && aligned_to(p.y[i], 16) && aligned_to(p.w[i], 16);
+  if (wide) {
+    const int per = cols > 2048 ? 2 : 1, rows_threads = ((cols / 8 + per - 1) / per + 31) / 32 * 32;
+#define BRANCH_ROWS(T)                                                                                                           \
+    if (per == 1) branch_join_rows_kernel<T, 1><<<static_cast<unsigned>(rows), rows_threads, 0, stream>>>(p);                    \
+    else branch_join_rows_kernel<T, 2><<<static_cast<unsigned>(rows), rows_threads, 0, stream>>>(p);
+    if (dtype == OSLO_DT_BF16) { BRANCH_ROWS(__nv_bfloat16) } else { BRANCH_ROWS(__half) }
+#undef BRANCH_ROWS
+    return static_cast<int>(cudaGetLastError());
+  }
 #define BRANCH_GO(V, N, THREADS)                                                                                 \
   {                                                                                                              \
     if (smem > 48 * 1024) {                                                                                      \

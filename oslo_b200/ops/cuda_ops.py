@@ -248,6 +248,42 @@ def fused_mlp(x: Tensor, w_in: Tensor, b_in: Optional[Tensor], w_out: Tensor, b_
     return _FusedMLP.apply(x, w_in, b_in, w_out, b_out, residual, reversed_)
 
 
+EMBED_GRAD_TOKENS = 32768
+
+
+class _Embedding(torch.autograd.Function):
+    """Lookup whose gradient goes row by row into the weight's own gradient (a flat buffer's view, see ``weight_grad``) or into one
+    zeroed tensor."""
+
+    @staticmethod
+    def forward(ctx, ids, weight):
+        ctx.save_for_backward(ids, weight)
+        return torch.nn.functional.embedding(ids, weight)
+
+    @staticmethod
+    def backward(ctx, dy):
+        ids, weight = ctx.saved_tensors
+        g = weight.grad
+        direct = (g is not None and getattr(weight, "_oslo_accum_grad", False) and g.dtype == weight.dtype and g.shape == weight.shape
+                  and g.is_contiguous() and g.data_ptr() % 16 == 0 and not torch.is_grad_enabled()
+                  and getattr(weight, "_oslo_grad_hook", None) is None)      # the data-parallel wrapper counts autograd's own calls here
+        if not direct:
+            g = torch.zeros_like(weight, memory_format=torch.contiguous_format)
+        d2 = dy.reshape(-1, dy.size(-1))
+        _ext().embedding_grad_(g, ids.reshape(-1).contiguous(), d2 if d2.is_contiguous() and d2.data_ptr() % 16 == 0 else d2.clone(memory_format=torch.contiguous_format))
+        return None, (None if direct else g)
+
+
+def embedding_ok(ids: Tensor, weight: Tensor) -> bool:
+    """Whether a lookup with a gradient takes ``_Embedding``."""
+    return (torch.is_grad_enabled() and weight.requires_grad and weight.is_cuda and ids.is_cuda and ids.dtype == torch.long
+            and weight.dtype in _16BIT and weight.dim() == 2 and weight.size(1) % 8 == 0 and 0 < ids.numel() <= EMBED_GRAD_TOKENS)
+
+
+def embedding(ids: Tensor, weight: Tensor) -> Tensor:
+    return _Embedding.apply(ids, weight)
+
+
 class _QKVLinear(torch.autograd.Function):
     """Three bias-free ``[out, in]`` projections of the same input. Forward is three GEMMs; the point is the
     backward: the three input-gradient GEMMs accumulate into one tensor in their epilogues instead of leaving two

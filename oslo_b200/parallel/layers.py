@@ -144,6 +144,13 @@ class StackedLinear(nn.Module):
 class Embedding(nn.Embedding):
     oslo_fused = False
 
+    def forward(self, ids: Tensor) -> Tensor:
+        if self.oslo_fused and ids.is_cuda and self.padding_idx is None and self.max_norm is None and not (self.scale_grad_by_freq or self.sparse):
+            from ..ops import cuda_ops, use_kernels
+            if use_kernels(ids) and cuda_ops.embedding_ok(ids, self.weight):
+                return cuda_ops.embedding(ids, self.weight)
+        return super().forward(ids)
+
 
 class VocabParallelEmbedding(nn.Embedding):
     """Embedding whose rows are split over the tensor-parallel group (``torch.chunk`` row ranges).

@@ -90,3 +90,46 @@ def test_gemm_tiles_cut_along_k(m, n, k, a_mn, b_mn, dtype):
         assert _rel(got, want) <= eps             # one rounding; GeLU's tanh is good to 2^-11
     y = co.gemm(a, b, a_mn, b_mn, flags=co.FLAG_OUT_FP32)
     assert _rel(y, z) <= 1e-5                     # 32-bit sums of k products: sqrt(8192) roundings of 2^-24, twice over
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("n, vocab, width, same", [(1, 5, 8, 0), (129, 50257, 768, 0), (4000, 300, 1032, 0), (5000, 1000, 2048, 3000), (8192, 50400, 4096, 0)])
+def test_embedding_gradient_by_rows(n, vocab, width, same, dtype):
+    """Sums in 32 bits and one rounding, ids repeated a few times, and one that fills more than a block's list."""
+    from oslo_b200.ops import cuda_ops as co
+    torch.manual_seed(n)
+    ids = torch.randint(0, vocab, (n,), device="cuda")
+    ids[torch.randperm(n, device="cuda")[:same]] = vocab // 2
+    w = torch.randn(vocab, width, device="cuda").to(dtype).requires_grad_()
+    dy = torch.randn(n, width, device="cuda").to(dtype)
+    out = co.embedding(ids.view(1, -1), w)
+    assert torch.equal(out[0], w.detach()[ids])
+    g, = torch.autograd.grad(out, w, dy[None])
+    want = torch.zeros(vocab, width, device="cuda", dtype=torch.float64).index_add_(0, ids, dy.double())
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    assert (g.double() - want).abs().max() <= eps * want.abs().max() + 1e-6 * max(same, 1)    # the second term: 32-bit sums of `same` rows
+    assert _rel(g, want) <= eps and not g[torch.bincount(ids, minlength=vocab) == 0].any()
+    held = torch.randn(vocab, width, device="cuda").to(dtype)
+    w.grad, w._oslo_accum_grad = held.clone(), True
+    co.embedding(ids.view(1, -1), w).backward(dy[None])
+    assert _rel(w.grad, held.double() + want) <= eps
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows", [296, 297, 1000])
+@pytest.mark.parametrize("cols, top", [(512, 1), (520, 3), (1024, 2), (2048, 3), (2056, 2), (4096, 5), (4104, 3)])
+def test_branch_join_rows(rows, cols, top, dtype):
+    """Both sides of the rule for whole rows in registers, against 64 bits: branches with and without a norm, gathered and scaled ones."""
+    from oslo_b200.ops import cuda_ops as co
+    from oslo_b200.ops.reference import Branch
+    torch.manual_seed(rows + cols)
+    mk = lambda *s: torch.randn(*s, device="cuda").to(dtype)  # noqa: E731
+    x, w1, w2, wn = torch.randn(rows, cols, device="cuda"), mk(cols), mk(cols), mk(cols)
+    slots = torch.randperm(rows * top + 5, device="cuda")[:rows * top].int().view(rows, top)
+    many, one, normed = mk(rows * top + 5, cols), mk(rows, cols + 8)[:, :cols], mk(rows, cols)
+    got, copies = co.branch_join(x, [Branch(many, slots=slots, top=top), Branch(one), Branch(normed, weight=wn, normed=True)], 0.5, 1e-5, [w1, w2])
+    d = normed.double()
+    z = x.double() + 0.5 * (many.double()[slots.long()].sum(1) + one.double() + d * torch.rsqrt(d.square().mean(-1, keepdim=True) + 1e-5) * wn.double())
+    r = torch.rsqrt(z.square().mean(-1, keepdim=True) + 1e-5)
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    assert _rel(got, z) <= 1e-6 and _rel(copies[0], z * r * w1.double()) <= eps and _rel(copies[1], z * r * w2.double()) <= eps
