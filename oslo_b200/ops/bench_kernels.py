@@ -246,7 +246,7 @@ def bench_mixers(args, timer: _Timer) -> None:
             if rows_n * t * h * d * 4 < 20e9:
                 kc, vc = mk(rows_n, h, t, d), mk(rows_n, h, t, d)
                 q3 = mk(rows_n, h, d)
-                report(case, f"decode {rows_n} attention (GPT-J, 2 launches)", lambda: ext.decode_attn(q3, kc, vc, lengths, d ** -0.5, 0),
+                report(case, f"decode {rows_n} attention (GPT-J)", lambda: ext.decode_attn(q3, kc, vc, lengths, d ** -0.5, 0),
                        gbytes=2 * rows_n * t * h * d * 2 / 1e9)
                 del kc, vc
             x, y, gate = torch.randn(rows_n, w, device="cuda"), mk(rows_n, w), mk(rows_n, w)
@@ -386,7 +386,7 @@ def bench_branches(args, timer: _Timer) -> None:
             del kc, vc
             if n * t * h * d * 4 < 20e9:
                 kf, vf = mk(n, h, t, d), mk(n, h, t, d)
-                report(case, tag + "attention (GPT-J, 2 launches)", lambda: ext.decode_attn(q3, kf, vf, lengths, d ** -0.5, 0), gbytes=2 * n * t * h * d * 2 / 1e9)
+                report(case, tag + "attention (GPT-J)", lambda: ext.decode_attn(q3, kf, vf, lengths, d ** -0.5, 0), gbytes=2 * n * t * h * d * 2 / 1e9)
                 del kf, vf
             xs, y1, y2, y3 = torch.randn(n, w, device="cuda"), mk(n, w), mk(n, w), mk(n, w)
             report(case, tag + "join, 3 branches, 2 normed", lambda: co.branch_join(xs, [(y1, vec, 0.5), (y2, vec, 0.5), (y3,)], 0.3, 1e-5, [vec, vec]),

@@ -266,7 +266,9 @@ class _Embedding(torch.autograd.Function):
         g = weight.grad
         direct = (g is not None and getattr(weight, "_oslo_accum_grad", False) and g.dtype == weight.dtype and g.shape == weight.shape
                   and g.is_contiguous() and g.data_ptr() % 16 == 0 and not torch.is_grad_enabled()
-                  and getattr(weight, "_oslo_grad_hook", None) is None)      # the data-parallel wrapper counts autograd's own calls here
+                  # the data-parallel wrapper and hooks of the user count autograd's own calls here
+                  and getattr(weight, "_oslo_grad_hook", None) is None and not weight._backward_hooks
+                  and not getattr(weight, "_post_accumulate_grad_hooks", None))
         if not direct:
             g = torch.zeros_like(weight, memory_format=torch.contiguous_format)
         d2 = dy.reshape(-1, dy.size(-1))
@@ -368,7 +370,7 @@ def small_rows_ok(x: Tensor, weight: Tensor, bias: Optional[Tensor], reversed_: 
     """Whether ``x W^T + b`` without gradients goes to the weight-streaming kernel: a few rows, k in 16-byte pieces, and any number of
     columns for ``[out, in]`` weights (GPT-2's head of 50257 words: 23 us through the library's product, floor 12), a multiple of 8
     for ``[in, out]``."""
-    if torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad):
+    if torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad or (bias is not None and bias.requires_grad)):
         return False
     k = x.size(-1)
     return (x.is_cuda and x.dtype in _16BIT and weight.dtype == x.dtype and k % 8 == 0 and 0 < x.numel() <= SMALL_M_ROWS * k
@@ -383,7 +385,7 @@ def few_rows(x: Tensor, weights, bias: Optional[Tensor] = None, gelu_from: int =
     if len({w.stride(0) for w in ws}) > 1:
         ws = [w.contiguous() for w in ws]
     k = x.size(-1)
-    y = _ext().few_rows(_as_operand(x.reshape(-1, k)), None, ws, int(reversed_), bias, int(gelu_from),
+    y = _ext().few_rows(_as_operand(x.reshape(-1, k)), None, ws, int(reversed_), None if bias is None else bias.contiguous(), int(gelu_from),
                         None if residual is None else _rows_of(residual),
                         None if ln is None else ln.weight, None if ln is None else ln.bias, 0.0 if ln is None else float(ln.eps))
     return y.view(*x.shape[:-1], y.size(-1))
@@ -599,7 +601,10 @@ def flash_attention(q: Tensor, k: Tensor, v: Tensor, causal: bool, window: Optio
 
 def decode_attention(q: Tensor, k_cache: Tensor, v_cache: Tensor, lengths: Tensor, scale: float,
                      window: Optional[int]) -> Tensor:
-    return _ext().decode_attn(q.contiguous(), k_cache, v_cache, lengths.to(torch.int32), float(scale), int(window or 0))
+    q = q.contiguous()
+    if q.data_ptr() % 16:
+        q = q.clone()
+    return _ext().decode_attn(q, k_cache, v_cache, lengths.to(torch.int32), float(scale), int(window or 0))
 
 
 class _FlashPacked(torch.autograd.Function):
