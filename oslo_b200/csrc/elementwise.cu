@@ -702,12 +702,12 @@ __global__ void __launch_bounds__(CS_WARPS * 32) ce_reduce_stats_kernel(const fl
 // bucket and a range of columns: it lists its tokens (every block reads all ids, which fit L2 many times over), then sums the rows of
 // each id. Bound by dy and the touched rows of grad; the library's gradient sorts the ids, sums segments through workspaces, fills a
 // whole [vocabulary, width] tensor and adds that to grad (50400 x 4096, 8192 tokens: 1.3 ms).
-constexpr int EG_THREADS = 128, EG_LIST = 2048;
+constexpr int EG_THREADS = 128, EG_LIST = 2048, EG_IDS = 8;
 template <typename T>
 __global__ void __launch_bounds__(EG_THREADS) embedding_grad_kernel(const long long* __restrict__ ids, const T* __restrict__ dy, T* __restrict__ grad,
                                                                     int n, long long vocab, int width, int buckets, int* err) {
   __shared__ int list_id[EG_LIST], list_t[EG_LIST];
-  __shared__ int count[EG_THREADS / 32 + 1];
+  __shared__ int count[EG_THREADS / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = (blockIdx.y * EG_THREADS + threadIdx.x) * 8;
   const bool live = c < width;
@@ -729,22 +729,33 @@ __global__ void __launch_bounds__(EG_THREADS) embedding_grad_kernel(const long l
     store_vec(g, v);
   };
   int total = 0;                                // tokens of this bucket, the same in every thread
-  for (int base = 0; base < n; base += EG_THREADS) {
-    const int t = base + threadIdx.x;
-    const long long id = t < n ? ids[t] : -1;
-    if (t < n && (id < 0 || id >= vocab) && blockIdx.x == 0 && blockIdx.y == 0) OSLO_REPORT_BOUNDS(err);   // no row to add to: skipped
-    const bool m = mine(id);
-    const unsigned vote = __ballot_sync(0xffffffffu, m);
-    if (!__syncthreads_or(vote != 0)) continue;
-    if (lane == 0) count[warp] = __popc(vote);
+  for (int base = 0; base < n; base += EG_THREADS * EG_IDS) {   // EG_IDS consecutive tokens per thread
+    unsigned hit = 0;
+#pragma unroll
+    for (int u = 0; u < EG_IDS; ++u) {
+      const int t = base + threadIdx.x * EG_IDS + u;
+      const long long id = t < n ? ids[t] : -1;
+      if (t < n && (id < 0 || id >= vocab) && blockIdx.x == 0 && blockIdx.y == 0) OSLO_REPORT_BOUNDS(err);   // no row to add to: skipped
+      hit |= (mine(id) ? 1u : 0u) << u;
+    }
+    int before = __popc(hit);                   // inclusive over the warp's lanes
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int o = __shfl_up_sync(0xffffffffu, before, off);
+      if (lane >= off) before += o;
+    }
     __syncthreads();
-    int at = total + __popc(vote & ((1u << lane) - 1));
+    if (lane == 31) count[warp] = before;
+    __syncthreads();
+    int at = total + before - __popc(hit);
     for (int w = 0; w < EG_THREADS / 32; ++w) {
       if (w < warp) at += count[w];
       total += count[w];
     }
-    if (m && at < EG_LIST) { list_id[at] = static_cast<int>(id); list_t[at] = t; }
-    __syncthreads();
+    for (; hit != 0; hit &= hit - 1, ++at) {
+      const int t = base + threadIdx.x * EG_IDS + __ffs(hit) - 1;
+      if (at < EG_LIST) { list_id[at] = static_cast<int>(ids[t]); list_t[at] = t; }
+    }
   }
   __syncthreads();
   if (total <= EG_LIST) {
