@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(128) causal_conv_kernel(const ConvParams p) {
       for (int i = 0; i < VEC; ++i) wr[j][i] = Num<T>::to(w[i * TAPS + j]);
 #pragma unroll
     for (int j = 0; j < TAPS - 1; ++j) input(t0 - TAPS + 1 + j, win[j + 1]);
-    constexpr int AHEAD = 8;                 // tokens whose inputs are on their way
+    constexpr int AHEAD = 4;                 // tokens whose inputs are on their way
     for (int tb = t0; tb < t1; tb += AHEAD) {
       float now[AHEAD][VEC];
 #pragma unroll
