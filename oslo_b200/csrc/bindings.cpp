@@ -131,7 +131,8 @@ Tensor gemm(const Tensor& a, const Tensor& b, int64_t a_mn, int64_t b_mn, const 
     ld_aux_out = static_cast<int>(aux_out->stride(0));
   }
   auto& st = dev_state(a.get_device());
-  const long long floats = oslo_gemm_split_floats(static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), usable_sms(st));
+  const int sms = usable_sms(st);          // read once: another thread may reserve SMs at any time
+  const long long floats = oslo_gemm_split_floats(static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), sms);
   Tensor ws;
   if (floats > 0) ws = at::empty({floats}, a.options().dtype(at::kFloat));
   const int rc = oslo_gemm_16bit(a.data_ptr(), b.data_ptr(), d.data_ptr(), static_cast<int>(M), static_cast<int>(N),
@@ -139,8 +140,8 @@ Tensor gemm(const Tensor& a, const Tensor& b, int64_t a_mn, int64_t b_mn, const 
                                  static_cast<int>(d.stride(0)), static_cast<int>(a_mn), static_cast<int>(b_mn),
                                  ptr_or_null(bias), ptr_or_null(aux), ld_aux,
                                  const_cast<void*>(ptr_or_null(aux_out)), ld_aux_out, fl, static_cast<float>(alpha),
-                                 floats > 0 ? ws.data_ptr<float>() : nullptr,
-                                 st.err.data_ptr<int>(), usable_sms(st), cur_stream(floats > 0 ? 2 : 1));
+                                 floats > 0 ? ws.data_ptr<float>() : nullptr, floats,
+                                 st.err.data_ptr<int>(), sms, cur_stream(floats > 0 ? 2 : 1));
   check_rc(rc, "gemm");
   return d;
 }

@@ -162,8 +162,10 @@ static int pair_split(int M, int N, int K, int num_sms) {
   return best;
 }
 
-// Tile shape selection, tensor maps and launch for a filled-in GemmParams (M, N, K, majors, flags, epilogue operands)
-static int dispatch_gemm(const void* A, const void* B, int lda, int ldb, GemmParams& p, int num_sms, cudaStream_t stream);
+// Tile shape selection, tensor maps and launch for a filled-in GemmParams (M, N, K, majors, flags, epilogue operands).
+// `split_floats`: what p.split_ws holds; tiles are cut along k only where it holds all of their ranges
+static int dispatch_gemm(const void* A, const void* B, int lda, int ldb, GemmParams& p, int num_sms, cudaStream_t stream,
+                         long long split_floats = 0);
 
 }  // namespace oslo
 
@@ -176,10 +178,17 @@ extern "C" long long oslo_gemm_split_floats(int M, int N, int K, int num_sms) {
   return s > 1 ? tiles % (num_sms / 2) * s * PAIR_TILE * PAIR_TILE : 0;
 }
 
+// ranges of k of the last wave's tiles in a launch on num_sms that was given `floats` of workspace: 1 (no cut) where that is too little,
+// as when it was sized for another number of SMs
+extern "C" int oslo_gemm_split_ranges(int M, int N, int K, int num_sms, long long floats) {
+  const long long need = oslo_gemm_split_floats(M, N, K, num_sms);
+  return need > 0 && need <= floats ? oslo::pair_split(M, N, K, num_sms) : 1;
+}
+
 extern "C" int oslo_gemm_16bit(const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb, int ldd,
                                int a_mn_major, int b_mn_major, const void* bias, const void* aux, int ld_aux,
-                               void* aux_out, int ld_aux_out, int flags, float alpha, float* split_ws, int* err_word,
-                               int num_sms, cudaStream_t stream) {
+                               void* aux_out, int ld_aux_out, int flags, float alpha, float* split_ws,
+                               long long split_floats, int* err_word, int num_sms, cudaStream_t stream) {
   using namespace oslo;
   if (M <= 0 || N <= 0 || K <= 0) return -1;
   if (flags & (GEMM_FLAG_CE_STATS | GEMM_FLAG_CE_GRAD | GEMM_FLAG_GLU)) return -7;   // those epilogues come through oslo_gemm_ce_16bit
@@ -189,7 +198,7 @@ extern "C" int oslo_gemm_16bit(const void* A, const void* B, void* D, int M, int
   p.a_mn_major = a_mn_major; p.b_mn_major = b_mn_major; p.flags = flags; p.alpha = alpha; p.err = err_word;
   p.split_ws = split_ws;
   p.comm = CommParams{};
-  return dispatch_gemm(A, B, lda, ldb, p, num_sms, stream);
+  return dispatch_gemm(A, B, lda, ldb, p, num_sms, stream, split_ws != nullptr ? split_floats : 0);
 }
 
 extern "C" int oslo_gemm_ce_16bit(const void* A, const void* B, int M, int N, int K, int lda, int ldb, int b_mn_major,
@@ -210,7 +219,8 @@ extern "C" int oslo_gemm_ce_16bit(const void* A, const void* B, int M, int N, in
 }
 
 namespace oslo {
-static int dispatch_gemm(const void* A, const void* B, int lda, int ldb, GemmParams& p, int num_sms, cudaStream_t stream) {
+static int dispatch_gemm(const void* A, const void* B, int lda, int ldb, GemmParams& p, int num_sms, cudaStream_t stream,
+                         long long split_floats) {
   const int M = p.M, N = p.N, K = p.K, a_mn_major = p.a_mn_major, b_mn_major = p.b_mn_major, flags = p.flags;
   // the tensor-map encoder is a driver-API call and needs the primary context bound to THIS thread; the
   // autograd engine's worker threads may not have made a runtime call yet
@@ -224,10 +234,8 @@ static int dispatch_gemm(const void* A, const void* B, int lda, int ldb, GemmPar
   // 4096 x 768, 48 tiles: 264, 298, 461), not with more (k = 8000, 768 x 3072, 36 tiles: 53.9, 60.0, 49.5), except where the idle ones
   // take ranges of k
   const long long pair_tiles = static_cast<long long>((M + PAIR_TILE - 1) / PAIR_TILE) * ((N + PAIR_TILE - 1) / PAIR_TILE);
-  if (p.split_ws != nullptr) {
-    p.split = pair_split(M, N, K, num_sms);
-    p.split_from = static_cast<int>(pair_tiles - pair_tiles % (num_sms / 2));
-  }
+  p.split = oslo_gemm_split_ranges(M, N, K, num_sms, split_floats);
+  p.split_from = static_cast<int>(pair_tiles - pair_tiles % (num_sms / 2));
   const bool pair = pair_enabled() && M >= PAIR_TILE && N >= PAIR_TILE && (pair_tiles >= num_sms / 4 + 1 || p.split > 1);
   const int bn = pair ? BM : (wide ? 256 : 128);   // B box rows: a pair's CTA stages 128 of the 256 tile columns
   CUtensorMap ta, tb;

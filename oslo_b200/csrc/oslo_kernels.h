@@ -31,9 +31,11 @@ extern "C" {
 
 int oslo_gemm_16bit(const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb, int ldd,
                     int a_mn_major, int b_mn_major, const void* bias, const void* aux, int ld_aux, void* aux_out,
-                    int ld_aux_out, int flags, float alpha, float* split_ws, int* err_word, int num_sms, cudaStream_t stream);
-// floats that split_ws has to hold (0: pass null)
-long long oslo_gemm_split_floats(int M, int N, int K, int num_sms);
+                    int ld_aux_out, int flags, float alpha, float* split_ws, long long split_floats, int* err_word, int num_sms,
+                    cudaStream_t stream);
+// floats that split_ws has to hold for tiles cut along k (0: pass null), and into how many ranges a launch with `floats` cuts them
+__attribute__((visibility("default"))) long long oslo_gemm_split_floats(int M, int N, int K, int num_sms);
+__attribute__((visibility("default"))) int oslo_gemm_split_ranges(int M, int N, int K, int num_sms, long long floats);
 
 // LM-head product with the cross-entropy pieces in its epilogue (x = A B^T + bias, never written as logits):
 //   mode 0 (GEMM_FLAG_CE_STATS): stats [ceil(N / 128), M, 3] fp32 records (max, sum exp, label logit or 0)
