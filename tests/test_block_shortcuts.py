@@ -1,0 +1,88 @@
+"""When a block of GPT-2 or GPT-Neo may compute what its modules compute without calling them, or call them with more than their
+input: on fake CUDA tensors, whose every Python branch runs. ``called`` records the calls of the layers' ``forward``."""
+import pytest
+import torch
+from torch._subclasses.fake_tensor import FakeTensorMode
+
+import oslo_b200 as ob
+from oslo_b200 import ops
+from oslo_b200.parallel import layers as L
+
+from .test_fake_cuda import _model
+
+KINDS = ["gpt2", "gpt_neo"]
+
+
+@pytest.fixture
+def kernels(monkeypatch):
+    if ops.load_ext() is None:
+        pytest.skip("extension not built")
+    monkeypatch.setattr(ops, "kernels_available", lambda: True)
+
+
+@pytest.fixture
+def called(monkeypatch):
+    seen = {}
+    for cls in (L.Conv1D, L.Linear):
+        def forward(self, x, activation=None, residual=None, _old=cls.forward):
+            seen[id(self)] = residual is not None
+            return _old(self, x, activation, residual)
+        monkeypatch.setattr(cls, "forward", forward)
+    return seen
+
+
+def _fused(kind):
+    cls, cfg = _model(kind)
+    if kind == "gpt2":
+        cfg.resid_pdrop = 0.0
+    with torch.device("cuda"):
+        model = cls._from_config(cfg, torch_dtype=torch.bfloat16)
+    return model.fuse()
+
+
+def _parts(model, kind):
+    block = model.transformer.h[0]
+    attn = block.attn if kind == "gpt2" else block.attn.attention
+    return block, attn, (attn.c_proj if kind == "gpt2" else attn.out_proj)
+
+
+def _ids():
+    return torch.zeros(2, 64, dtype=torch.long, device="cuda")
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_layers_nobody_listens_to_are_not_called(kernels, called, kind):
+    with FakeTensorMode():
+        model = _fused(kind).train()
+        block, attn, out_proj = _parts(model, kind)
+        model(input_ids=_ids())
+        assert id(block.mlp.c_fc) not in called and called[id(out_proj)]
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("register", ["register_full_backward_hook", "register_full_backward_pre_hook"])
+@pytest.mark.parametrize("name", ["mlp", "mlp.c_fc", "mlp.c_proj", "attn.attention.q_proj"])
+def test_a_backward_hook_has_its_module_called(kernels, called, kind, register, name):
+    with FakeTensorMode():
+        model = _fused(kind).train()
+        block, _, _ = _parts(model, kind)
+        if name.startswith("attn.attention") and kind == "gpt2":
+            pytest.skip("GPT-Neo's layers")
+        getattr(block.get_submodule(name), register)(lambda *a: None)
+        model(input_ids=_ids())
+        layer = block.mlp.c_fc if name == "mlp" else block.get_submodule(name)
+        assert id(layer) in called
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("register", ["register_module_full_backward_hook", "register_module_full_backward_pre_hook"])
+def test_a_global_backward_hook_has_all_modules_called(kernels, called, kind, register):
+    with FakeTensorMode():
+        model = _fused(kind).train()
+        block, _, _ = _parts(model, kind)
+        handle = getattr(torch.nn.modules.module, register)(lambda *a: None)
+        try:
+            model(input_ids=_ids())
+        finally:
+            handle.remove()
+        assert id(block.mlp.c_fc) in called
