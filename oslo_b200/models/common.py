@@ -273,7 +273,8 @@ def unhooked(*modules: nn.Module) -> bool:
 
 def residual_inside(block, attn, mlp, out_proj, fc_in, fc_out, hidden_states: Tensor, kw) -> bool:
     """Whether a pre-norm block's two residual additions run inside GEMM epilogues, and its MLP as one autograd node: plain fused layers
-    on a CUDA input of the large-input path, and no dropout in between."""
+    on a CUDA input of the large-input path, and no dropout in between. Attention (``block.attn``, ``attn`` inside it) and its output
+    projection then return attention plus the residual stream, so nobody may listen to them."""
     if not (hidden_states.is_cuda and attn.fused and mlp.fused and mlp.activation in GELU_TANH_NAMES and kw.get("seq_shape") is None
             and type(out_proj) is type(fc_in) is type(fc_out) and not (block.training and (attn.resid_pdrop or mlp.resid_pdrop))):
         return False
@@ -282,7 +283,7 @@ def residual_inside(block, attn, mlp, out_proj, fc_in, fc_out, hidden_states: Te
     from ..parallel.layers import Conv1D, Linear
     kind = type(fc_out)
     return (kind in (Conv1D, Linear) and get_config().block_fusion and all(m.oslo_fused for m in (out_proj, fc_in, fc_out))
-            and unhooked(mlp, fc_in, fc_out)
+            and unhooked(block.attn, attn, mlp, out_proj, fc_in, fc_out)
             and all(m.bias is None or m.bias.dtype == hidden_states.dtype for m in (fc_in, fc_out))
             and cuda_ops.fused_mlp_ok(hidden_states, fc_in.weight, fc_out.weight, kind is Conv1D))
 

@@ -86,3 +86,17 @@ def test_a_global_backward_hook_has_all_modules_called(kernels, called, kind, re
         finally:
             handle.remove()
         assert id(block.mlp.c_fc) in called
+
+
+@pytest.mark.parametrize("train", [True, False])
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("where", ["attn", "attention", "out_proj"])
+def test_a_hook_on_attention_gets_the_attention_alone(kernels, called, kind, where, train):
+    """The residual stream is not added inside modules whose output somebody takes or replaces."""
+    with FakeTensorMode():
+        model = _fused(kind).train(train)
+        block, attn, out_proj = _parts(model, kind)
+        {"attn": block.attn, "attention": attn, "out_proj": out_proj}[where].register_forward_hook(lambda *a: None)
+        with torch.set_grad_enabled(train):
+            model(input_ids=_ids())
+        assert called[id(out_proj)] is False
