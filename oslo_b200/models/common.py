@@ -265,10 +265,11 @@ class AttentionCore(nn.Module):
 
 def unhooked(*modules: nn.Module) -> bool:
     """Whether a block may compute what these modules compute without calling them: nobody listens to their calls, forward or
-    backward."""
+    backward, and none has a ``forward`` of its own. Their classes are the caller's to check: a subclass computes what it likes."""
     g = nn.modules.module
     return not (g._global_forward_hooks or g._global_forward_pre_hooks or g._global_backward_hooks or g._global_backward_pre_hooks
-                or any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks for m in modules))
+                or any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in vars(m)
+                       for m in modules))
 
 
 def residual_inside(block, attn, mlp, out_proj, fc_in, fc_out, hidden_states: Tensor, kw) -> bool:

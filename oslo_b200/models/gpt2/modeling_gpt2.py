@@ -180,16 +180,15 @@ class GPT2Block(nn.Module):
         self.mlp = GPT2MLP(inner, config)
 
     def forward(self, hidden_states: Tensor, encoder_hidden_states=None, encoder_attention_mask=None, **kw):
-        if encoder_hidden_states is None and kw.get("cache") is not None:
-            attn, mlp = self.attn, self.mlp
+        attn, mlp = self.attn, self.mlp
+        own = encoder_hidden_states is None and type(attn) is FusedGPT2Attention and type(mlp) is FusedGPT2MLP
+        if own and kw.get("cache") is not None:
             fast = decode_block(self, attn, mlp, (attn.c_attn,), attn.c_proj, mlp.c_fc, mlp.c_proj, hidden_states, kw)
             if fast is not None:
                 return fast, None, None
-        if encoder_hidden_states is None and residual_inside(self, self.attn, self.mlp, self.attn.c_proj, self.mlp.c_fc, self.mlp.c_proj,
-                                                             hidden_states, kw):
+        if own and residual_inside(self, attn, mlp, attn.c_proj, mlp.c_fc, mlp.c_proj, hidden_states, kw):
             from ...ops import cuda_ops
-            mlp = self.mlp
-            hidden_states, present, probs = self.attn(self.ln_1(hidden_states), residual=hidden_states, **kw)
+            hidden_states, present, probs = attn(self.ln_1(hidden_states), residual=hidden_states, **kw)
             return cuda_ops.fused_mlp(self.ln_2(hidden_states), mlp.c_fc.weight, mlp.c_fc.bias, mlp.c_proj.weight, mlp.c_proj.bias,
                                       hidden_states, True), present, probs
         a, present, probs = self.attn(self.ln_1(hidden_states), **kw)

@@ -161,14 +161,15 @@ class GPTNeoBlock(nn.Module):
         self.mlp = GPTNeoMLP(inner, config)
 
     def forward(self, hidden_states: Tensor, **kw):
-        if kw.get("cache") is not None and unhooked(self.attn):
-            attn, mlp = self.attn.attention, self.mlp
+        attn = self.attn.attention if type(self.attn) is GPTNeoAttention else None
+        mlp = self.mlp
+        own = type(attn) in (FusedGPTNeoSelfAttention, FusedGPTNeoLocalSelfAttention) and type(mlp) is FusedGPTNeoMLP
+        if own and kw.get("cache") is not None and unhooked(self.attn):
             fast = decode_block(self, attn, mlp, (attn.q_proj, attn.k_proj, attn.v_proj), attn.out_proj, mlp.c_fc, mlp.c_proj,
                                 hidden_states, kw)
             if fast is not None:
                 return fast, None, None
-        attn, mlp = self.attn.attention, self.mlp
-        if residual_inside(self, attn, mlp, attn.out_proj, mlp.c_fc, mlp.c_proj, hidden_states, kw):
+        if own and residual_inside(self, attn, mlp, attn.out_proj, mlp.c_fc, mlp.c_proj, hidden_states, kw):
             from ...ops import cuda_ops
             hidden_states, present, probs = self.attn(self.ln_1(hidden_states), residual=hidden_states, **kw)
             return cuda_ops.fused_mlp(self.ln_2(hidden_states), mlp.c_fc.weight, mlp.c_fc.bias, mlp.c_proj.weight, mlp.c_proj.bias,

@@ -100,3 +100,64 @@ def test_a_hook_on_attention_gets_the_attention_alone(kernels, called, kind, whe
         with torch.set_grad_enabled(train):
             model(input_ids=_ids())
         assert called[id(out_proj)] is False
+
+
+class _OwnAttention(torch.nn.Module):
+    """A user's attention: its own signature, none of the attributes of the family's."""
+
+    def forward(self, hidden_states, layer_past=None, attention_mask=None, position_ids=None, head_mask=None, use_cache=False,
+                output_attentions=False, cache=None, layer_id=0, seq_shape=None):
+        return 2 * hidden_states, None, None
+
+
+@pytest.mark.parametrize("device", ["cpu", "cuda"])
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("part", ["mlp", "attn"])
+def test_a_part_of_the_users_own_is_called(kernels, kind, device, part):
+    from oslo_b200.models.common import StaticKVCache
+    cls, cfg = _model(kind)
+    with FakeTensorMode():
+        with torch.device(device):
+            model = cls._from_config(cfg, torch_dtype=torch.bfloat16)
+        if device == "cuda":
+            model.fuse()
+        model.eval()
+        for block in model.transformer.h:
+            setattr(block, part, torch.nn.SiLU() if part == "mlp" else _OwnAttention())
+        ids = _ids().to(device)
+        for kw in ({}, {"past_key_values": StaticKVCache(100)})[:2 if part == "mlp" else 1]:     # this attention fills no cache
+            with torch.no_grad():
+                assert model(input_ids=ids, use_cache=bool(kw), **kw).logits.shape[:2] == (2, 64)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("how", ["mlp class", "mlp forward", "c_fc forward", "attention class", "attention forward", "out_proj forward"])
+def test_overridden_modules_are_called(kernels, called, kind, how):
+    """Subclasses of the family's modules, and modules with a ``forward`` of their own, in a prompt and in a step on device positions."""
+    from oslo_b200.models.common import StaticKVCache
+    with FakeTensorMode():
+        model = _fused(kind).eval()
+        seen = []
+        for block in model.transformer.h:
+            attn = block.attn if kind == "gpt2" else block.attn.attention
+            out_proj = attn.c_proj if kind == "gpt2" else attn.out_proj
+            target = {"mlp": block.mlp, "c_fc": block.mlp.c_fc, "attention": attn, "out_proj": out_proj}[how.split()[0]]
+            if how.endswith("class"):
+                base = type(target)
+
+                def forward(self, x, _base=base, **kw):
+                    seen.append(kw.get("residual"))
+                    return _base.forward(self, x, **kw)
+                target.__class__ = type("Own", (base,), {"forward": forward})
+            else:
+                def forward(x, _old=target.forward, **kw):
+                    seen.append(kw.get("residual"))
+                    return _old(x, **kw)
+                target.forward = forward
+        with torch.no_grad():
+            cache = StaticKVCache(100)
+            model(input_ids=_ids(), past_key_values=cache, use_cache=True)
+            assert len(seen) == len(model.transformer.h)
+            cache.use_device_positions()
+            model(input_ids=_ids()[:, :1], past_key_values=cache, use_cache=True)
+        assert len(seen) == 2 * len(model.transformer.h) and all(r is None for r in seen)
