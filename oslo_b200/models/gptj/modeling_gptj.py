@@ -291,7 +291,9 @@ class GPTJBlock(nn.Module):
                               mlp.fc_in.bias, attn.q_proj.mpu)
 
     def forward(self, hidden_states: Tensor, **kw):
-        fold = hidden_states.is_cuda and self._fold_ln(hidden_states)
+        cache = kw.get("cache")
+        fold = (cache is not None and getattr(cache, "device_positions", False) and hidden_states.size(1) == 1      # else no _decode_step
+                and hidden_states.is_cuda and self._fold_ln(hidden_states))
         packed = self._packed_decode_projections(hidden_states, self.ln_1) if fold else None
         x = hidden_states if packed is not None else self.ln_1(hidden_states)
         if packed is None and x.is_cuda and not fold:
@@ -300,6 +302,8 @@ class GPTJBlock(nn.Module):
             fast = self._decode_step(hidden_states, packed, kw)
             if fast is not None:
                 return fast
+            if fold:
+                x = self.ln_1(hidden_states)
             a, present, probs = self.attn(x, qkv=packed[:3], **kw)
             m = self.mlp(x, h=packed[3])
             return a + m + hidden_states, present, probs

@@ -161,3 +161,30 @@ def test_overridden_modules_are_called(kernels, called, kind, how):
             cache.use_device_positions()
             model(input_ids=_ids()[:, :1], past_key_values=cache, use_cache=True)
         assert len(seen) == 2 * len(model.transformer.h) and all(r is None for r in seen)
+
+
+@pytest.mark.parametrize("step", [False, True])
+def test_gptj_attention_and_mlp_get_the_normed_stream(kernels, monkeypatch, step):
+    """Few rows whose q, k, v and first MLP layer are one product, outside the whole-block step: attention and MLP are called, and
+    with what the norm returned."""
+    from oslo_b200.models.common import StaticKVCache
+    normed, got = [], []
+    old = L.LayerNorm.forward
+    monkeypatch.setattr(L.LayerNorm, "forward", lambda self, x: normed.append(old(self, x)) or normed[-1])
+    cls, cfg = _model("gptj")
+    with FakeTensorMode():
+        with torch.device("cuda"):
+            model = cls._from_config(cfg, torch_dtype=torch.bfloat16)
+        model.fuse().eval()
+        ids, cache = torch.zeros(2, 16 if not step else 1, dtype=torch.long, device="cuda"), StaticKVCache(100)
+        with torch.no_grad():
+            if step:       # a step whose keys are masked
+                model(input_ids=ids, past_key_values=cache, use_cache=True)
+                cache.use_device_positions()
+            for block in model.transformer.h:
+                for m in (block.attn, block.mlp):
+                    m.register_forward_pre_hook(lambda m, args: got.append(args[0]))
+            normed.clear()
+            model(input_ids=ids, past_key_values=cache, use_cache=True,
+                  **({"attention_mask": torch.ones(2, 2, dtype=torch.long, device="cuda")} if step else {}))
+    assert len(got) == 4 and all(any(g is n for n in normed) for g in got)
