@@ -176,7 +176,7 @@ def test_gptj_attention_and_mlp_get_the_normed_stream(kernels, monkeypatch, step
         with torch.device("cuda"):
             model = cls._from_config(cfg, torch_dtype=torch.bfloat16)
         model.fuse().eval()
-        ids, cache = torch.zeros(2, 16 if not step else 1, dtype=torch.long, device="cuda"), StaticKVCache(100)
+        ids, cache = torch.zeros(2, 4 if not step else 1, dtype=torch.long, device="cuda"), StaticKVCache(100)
         with torch.no_grad():
             if step:       # a step whose keys are masked
                 model(input_ids=ids, past_key_values=cache, use_cache=True)
