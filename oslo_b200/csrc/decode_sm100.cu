@@ -107,6 +107,7 @@ __global__ void __launch_bounds__(256) prompt_append_kernel(const V* __restrict_
 // own pieces of K and V with cp.async, DA_STAGES - 1 batches of DA_KEYS keys ahead: shared memory is a private queue, without barriers,
 // and keeps up to 128 KB per SM on their way. With `k` given, the new token's key and value are rotated (the first rotary_dim
 // dims), written to the cache at write_index[0] by the first split, and taken from registers by whichever split reaches that position.
+// A write_index outside the cache writes nothing, makes the result NaN and sets the error word.
 struct DecodeAttn {
   const void* q; const void* k; const void* v;          // [B, H, D] by strides (b, h); k, v may be null
   void* kc; void* vc; void* o;                          // caches [B, H, T, D], result [B, H, D]
@@ -185,10 +186,12 @@ __global__ void __launch_bounds__(DA_WARPS * 32, 4) decode_attn_kernel(const Dec
   const T* kb = reinterpret_cast<const T*>(p.kc) + head + d0;
   const T* vb = reinterpret_cast<const T*>(p.vc) + head + d0;
   int wi = -1;
+  bool lost = false;                            // a token that has no place in the cache
   if (p.k != nullptr) {
     const long long at = p.write_index[0];
-    if (at < 0 || at >= p.T) OSLO_REPORT_BOUNDS(p.err);   // never write outside the cache
-    else wi = static_cast<int>(at);
+    lost = at < 0 || at >= p.T;
+    if (!lost) wi = static_cast<int>(at);
+    else if (threadIdx.x == 0 && p.err != nullptr) atomicCAS(p.err, 0, ERR_BOUNDS);   // in every build: a replayed step has no host to refuse it
   }
   const uint32_t ring = smem_u32(da_smem) + (w * (2 * KB * 32) + l) * 16;
   int ft = t0 + w * BATCH, fslot = 0;
@@ -232,7 +235,7 @@ __global__ void __launch_bounds__(DA_WARPS * 32, 4) decode_attn_kernel(const Dec
   float q[8];
   dec_unpack<T>(qraw, q);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) q[i] *= p.scale * DA_LOG2E;
+  for (int i = 0; i < 8; ++i) q[i] *= lost ? CUDART_NAN_F : p.scale * DA_LOG2E;   // no answer from the keys that are left
   float m = -CUDART_INF_F, s = 0.f, acc[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc[i] = 0.f;

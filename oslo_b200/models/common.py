@@ -53,7 +53,8 @@ class StaticKVCache:
 
     def use_device_positions(self, on: bool = True) -> None:
         """Keep the write position of single-token appends on the device (needs one prior append). The position
-        tensor is allocated once and updated in place, so a CUDA graph captured earlier keeps addressing it."""
+        tensor is allocated once and updated in place, so a CUDA graph captured earlier keeps addressing it. A captured step that is
+        replayed past ``max_len`` writes nothing: its attention is NaN and ``ops.cuda_ops.device_error_code`` is 6 from then on."""
         if not on:
             self.device_positions = False
             return

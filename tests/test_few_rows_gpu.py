@@ -79,6 +79,42 @@ def test_decode_step_attention(dtype, d, rotary, b, h, t, at, window):
     torch.testing.assert_close(cuda_ops.decode_attention(q, k2, v2, lengths, d ** -0.5, window or None).double(), ref, atol=3 * EPS[dtype], rtol=3 * EPS[dtype])
 
 
+@pytest.mark.parametrize("kind", ["gpt2", "gpt_neo", "gptj"])
+def test_a_step_replayed_past_the_end_of_the_cache_is_refused(kind):
+    """A captured step of the user's own, one replay too many: no finite logits, nothing written, and the device's error word says so."""
+    from oslo_b200.models.common import StaticKVCache
+    from oslo_b200.ops import cuda_ops
+    if kind == "gpt2":
+        model = ob.GPT2LMHeadModel(ob.GPT2Config(vocab_size=64, n_positions=64, n_embd=64, n_layer=2, n_head=2))
+    elif kind == "gpt_neo":
+        model = ob.GPTNeoForCausalLM(ob.GPTNeoConfig(vocab_size=64, max_position_embeddings=64, hidden_size=64, num_layers=2, num_heads=2,
+                                                     window_size=4, attention_types=[[["global", "local"], 1]]))
+    else:
+        model = ob.GPTJForCausalLM(ob.GPTJConfig(vocab_size=64, n_positions=64, n_embd=64, n_layer=2, n_head=2, rotary_dim=16))
+    model = model.to("cuda", torch.bfloat16).fuse().eval()
+    ids, cache = torch.zeros(3, 6, dtype=torch.long, device="cuda"), StaticKVCache(8)
+    step = lambda: model(input_ids=ids[:, :1], past_key_values=cache, position_ids=cache.lengths_dev.long()[:, None], use_cache=True).logits  # noqa: E731
+    with torch.no_grad():
+        model(input_ids=ids, past_key_values=cache, use_cache=True)
+        cache.use_device_positions()
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            step()                                    # the first of two places
+        torch.cuda.current_stream().wait_stream(side)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = step()
+    cuda_ops.reset_device_error(ids)
+    graph.replay()
+    assert torch.isfinite(out).all() and cuda_ops.device_error_code(ids) == 0
+    held = [t.clone() for t in (*cache.k.values(), *cache.v.values())]
+    graph.replay()
+    assert not torch.isfinite(out).any() and cuda_ops.device_error_code(ids) == 6
+    assert all(torch.equal(a, b) for a, b in zip(held, (*cache.k.values(), *cache.v.values())))
+    cuda_ops.reset_device_error(ids)
+
+
 @pytest.mark.parametrize("b, h, s, d, t, start", [(1, 1, 1, 8, 1, 0), (2, 3, 17, 64, 40, 5), (4, 16, 200, 256, 210, 10), (3, 5, 333, 80, 333, 0)])
 def test_prompt_append(b, h, s, d, t, start):
     """Keys and values of a prompt land where slice copies put them, from slices of joint rows and from contiguous tensors."""
