@@ -245,9 +245,9 @@ class AttentionCore(nn.Module):
         if cache is not None:
             if (cache.device_positions and q.size(2) == 1 and self.fused and q.is_cuda and key_padding_mask is None
                     and not output_attentions and head_mask is None):
-                from ..ops import cuda_ops
+                from ..ops import cuda_ops, use_kernels
                 kc, vc = cache.kv_storage(layer_id, k.size(0), k.size(1), k.size(3), v.size(3), k.dtype, k.device, 1)
-                if cuda_ops.decode_step_ok(q[:, :, 0], kc, vc):      # append and attention in one kernel
+                if use_kernels(q) and cuda_ops.decode_step_ok(q[:, :, 0], kc, vc):      # append and attention in one kernel
                     out = cuda_ops.decode_step_attention(q[:, :, 0], k[:, :, 0], v[:, :, 0], kc, vc, cache.lengths_next,
                                                          cache.lengths_dev, cache.write_index, self.scale, self.window)
                     return out.unsqueeze(2), None, None
@@ -281,10 +281,10 @@ def residual_inside(block, attn, mlp, out_proj, fc_in, fc_out, hidden_states: Te
             and type(out_proj) is type(fc_in) is type(fc_out) and not (block.training and (attn.resid_pdrop or mlp.resid_pdrop))):
         return False
     from ..config import get_config
-    from ..ops import cuda_ops
+    from ..ops import cuda_ops, use_kernels
     from ..parallel.layers import Conv1D, Linear
     kind = type(fc_out)
-    return (kind in (Conv1D, Linear) and get_config().block_fusion and all(m.oslo_fused for m in (out_proj, fc_in, fc_out))
+    return (use_kernels(hidden_states) and kind in (Conv1D, Linear) and get_config().block_fusion and all(m.oslo_fused for m in (out_proj, fc_in, fc_out))
             and unhooked(block.attn, attn, mlp, out_proj, fc_in, fc_out)
             and all(m.bias is None or m.bias.dtype == hidden_states.dtype for m in (fc_in, fc_out))
             and cuda_ops.fused_mlp_ok(hidden_states, fc_in.weight, fc_out.weight, kind is Conv1D))
@@ -302,8 +302,10 @@ def decode_block(block, attn, mlp, qkv, out_proj, fc_in, fc_out, hidden_states: 
             or any(kw.get(name) is not None for name in ("attention_mask", "head_mask", "seq_shape", "layer_past"))
             or kw.get("output_attentions")):
         return None
-    from ..ops import cuda_ops
+    from ..ops import cuda_ops, use_kernels
     from ..parallel.layers import Conv1D, LayerNorm, Linear
+    if not use_kernels(hidden_states):
+        return None
     layers = (*qkv, out_proj, fc_in, fc_out)
     kind = Conv1D if len(qkv) == 1 else Linear
     if not (all(type(m) is kind and m.oslo_fused for m in layers) and all(type(m) is LayerNorm and m.oslo_fused for m in (block.ln_1, block.ln_2))

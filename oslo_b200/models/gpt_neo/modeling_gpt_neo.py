@@ -93,8 +93,8 @@ class GPTNeoSelfAttention(AttentionCore):
         layers = (self.q_proj, self.k_proj, self.v_proj)
         if (self.fused and x.is_cuda and all(type(l) is Linear and l.oslo_fused and l.bias is None for l in layers)
                 and unhooked(*layers) and get_config().block_fusion):
-            from ...ops import cuda_ops
-            if cuda_ops.qkv_linear_ok(x, *(l.weight for l in layers)):
+            from ...ops import cuda_ops, use_kernels
+            if use_kernels(x) and cuda_ops.qkv_linear_ok(x, *(l.weight for l in layers)):
                 return cuda_ops.qkv_linear(x, *(l.weight for l in layers))
         return tuple(l(x) for l in layers)
 

@@ -24,7 +24,7 @@ _GELU_NAMES = ("gelu", "gelu_new", "gelu_tanh", "gelu_pytorch_tanh")
 
 def _linear(x: Tensor, weight: Tensor, bias: Optional[Tensor], reversed: bool, fused: bool,
             activation: Optional[str] = None, residual: Optional[Tensor] = None) -> Tensor:
-    if fused and residual is not None and x.is_cuda:
+    if fused and residual is not None and ops.use_kernels(x):
         from ..ops import cuda_ops
         return cuda_ops.linear(x, weight, bias, reversed, activation, residual)
     y = ops.linear(x, weight, bias, reversed, activation) if fused else ops.reference.linear(x, weight, bias, reversed, activation)

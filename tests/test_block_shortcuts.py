@@ -188,3 +188,27 @@ def test_gptj_attention_and_mlp_get_the_normed_stream(kernels, monkeypatch, step
             model(input_ids=ids, past_key_values=cache, use_cache=True,
                   **({"attention_mask": torch.ones(2, 2, dtype=torch.long, device="cuda")} if step else {}))
     assert len(got) == 4 and all(any(g is n for n in normed) for g in got)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_without_the_extension_the_fallback_runs(monkeypatch, kind):
+    """``OSLO_B200_ALLOW_FALLBACK=1``: prompt, step on device positions and training through the PyTorch statements."""
+    from oslo_b200.models.common import StaticKVCache
+    from oslo_b200.ops import cuda_ops
+
+    def load_ext(required=False):
+        if required:
+            raise RuntimeError("CUDA extension unavailable")
+    monkeypatch.setattr(ops, "load_ext", load_ext)
+    monkeypatch.setattr(cuda_ops, "load_ext", load_ext)
+    monkeypatch.setenv("OSLO_B200_ALLOW_FALLBACK", "1")
+    with FakeTensorMode():
+        model = _fused(kind).eval()
+        cache = StaticKVCache(100)
+        with torch.no_grad():
+            model(input_ids=_ids(), past_key_values=cache, use_cache=True)
+            cache.use_device_positions()
+            assert model(input_ids=_ids()[:, :1], past_key_values=cache, use_cache=True).logits.shape[:2] == (2, 1)
+        assert model.train()(input_ids=_ids(), labels=_ids()).loss.shape == ()
+        x = torch.zeros(2, 1, 512, device="cuda", dtype=torch.bfloat16)
+        assert model.transformer.h[0].mlp.c_proj(x.new_zeros(2, 100, 2048), residual=x.new_zeros(2, 100, 512)).shape == (2, 100, 512)
