@@ -257,13 +257,20 @@ class GPTJBlock(nn.Module):
         mpu = getattr(attn.out_proj, "mpu", None)
         tp = mpu.tp if mpu is not None else 1
         fc_bias = mlp.fc_out.bias
-        # bias and residual enter the sum exactly once: on tensor-parallel rank 0, before the all-reduce
-        first = tp == 1 or mpu.tp_rank == 0
+        # bias and residual enter the sum exactly once. Tensor parallel, up to 4 rows: on rank 0, inside the product (launches count
+        # there); more rows: after the all-reduce, so that no part is rounded to 16 bits at the residual stream's magnitude
+        inside = tp == 1 or rows <= 4
+        first = inside and (tp == 1 or mpu.tp_rank == 0)
         z = cuda_ops.gemv_two_inputs(o.reshape(rows, -1), h, self._packed2_w, fc_bias if first else None,
                                      hidden_states.reshape(rows, -1) if first else None)
         if tp > 1:
             z = mpu._reduce(z)
-        return z.view_as(hidden_states), None, None
+        z = z.view_as(hidden_states)
+        if not inside:
+            if fc_bias is not None:
+                z = z + fc_bias
+            z = z + hidden_states
+        return z, None, None
 
     def _tp_shared_input(self, x: Tensor):
         """``(q, k, v, h)`` through ``fused_tp.tp_block_input`` when the four layers are plain column-parallel shards

@@ -212,3 +212,33 @@ def test_without_the_extension_the_fallback_runs(monkeypatch, kind):
         assert model.train()(input_ids=_ids(), labels=_ids()).loss.shape == ()
         x = torch.zeros(2, 1, 512, device="cuda", dtype=torch.bfloat16)
         assert model.transformer.h[0].mlp.c_proj(x.new_zeros(2, 100, 2048), residual=x.new_zeros(2, 100, 512)).shape == (2, 100, 512)
+
+
+@pytest.mark.parametrize("rows", [4, 5, 64])
+@pytest.mark.parametrize("rank", [0, 1])
+def test_gptj_tensor_parallel_step_adds_the_residual_after_the_reduction(kernels, monkeypatch, rows, rank):
+    """More than 4 rows: the parts that are summed over the ranks are products alone."""
+    from types import SimpleNamespace
+
+    from oslo_b200.models.common import StaticKVCache
+    from oslo_b200.ops import cuda_ops
+    products, reduced = [], []
+    old = cuda_ops.gemv_two_inputs
+    monkeypatch.setattr(cuda_ops, "gemv_two_inputs", lambda *a: products.append((a[3], a[4], old(*a))) or products[-1][2])
+    mpu = SimpleNamespace(tp=2, tp_rank=rank, _reduce=lambda z: reduced.append(z) or z)
+    cls, cfg = _model("gptj")
+    with FakeTensorMode():
+        with torch.device("cuda"):
+            model = cls._from_config(cfg, torch_dtype=torch.bfloat16)
+        model.fuse().eval()
+        ids, cache = torch.zeros(rows, 8, dtype=torch.long, device="cuda"), StaticKVCache(100)
+        with torch.no_grad():
+            model(input_ids=ids, past_key_values=cache, use_cache=True)
+            cache.use_device_positions()
+            for block in model.transformer.h:
+                block.attn.out_proj.mpu = mpu
+            assert model(input_ids=ids[:, :1], past_key_values=cache, use_cache=True).logits.shape[0] == rows
+    assert len(products) == len(reduced) == len(model.transformer.h)
+    inside = rows <= 4 and rank == 0
+    for (bias, residual, y), z in zip(products, reduced):
+        assert (bias is not None) == inside and (residual is not None) == inside and z is y
