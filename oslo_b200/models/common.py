@@ -273,6 +273,17 @@ def unhooked(*modules: nn.Module) -> bool:
                        for m in modules))
 
 
+def learns(ln: nn.LayerNorm) -> bool:
+    return torch.is_grad_enabled() and any(p.requires_grad for p in ln.parameters())
+
+
+def foldable_norm(ln: nn.LayerNorm, x: Tensor) -> bool:
+    """Whether the kernel that multiplies the few rows ``x`` can compute their LayerNorm on the way (it has no backward)."""
+    from ..ops import cuda_ops
+    return (ln.weight is not None and ln.weight.dtype == x.dtype and ln.weight.numel() == x.size(-1)
+            and (ln.bias is None or ln.bias.dtype == x.dtype) and cuda_ops.folded_ln_ok(x) and not learns(ln))
+
+
 def residual_inside(block, attn, mlp, out_proj, fc_in, fc_out, hidden_states: Tensor, kw) -> bool:
     """Whether a pre-norm block's two residual additions run inside GEMM epilogues, and its MLP as one autograd node: plain fused layers
     on a CUDA input of the large-input path, and no dropout in between. Attention (``block.attn``, ``attn`` inside it) and its output
@@ -309,7 +320,7 @@ def decode_block(block, attn, mlp, qkv, out_proj, fc_in, fc_out, hidden_states: 
     layers = (*qkv, out_proj, fc_in, fc_out)
     kind = Conv1D if len(qkv) == 1 else Linear
     if not (all(type(m) is kind and m.oslo_fused for m in layers) and all(type(m) is LayerNorm and m.oslo_fused for m in (block.ln_1, block.ln_2))
-            and unhooked(attn, mlp, block.ln_1, block.ln_2, *layers)):
+            and unhooked(attn, mlp, block.ln_1, block.ln_2, *layers)) or learns(block.ln_1) or learns(block.ln_2):
         return None
     kn = kind is Conv1D
     x = hidden_states
@@ -324,7 +335,7 @@ def decode_block(block, attn, mlp, qkv, out_proj, fc_in, fc_out, hidden_states: 
         return None
 
     def normed(h, ln, weights, bias, gelu_from):
-        if cuda_ops.folded_ln_ok(h) and ln.weight is not None and ln.weight.dtype == h.dtype:
+        if foldable_norm(ln, h):
             return cuda_ops.few_rows(h, weights, bias, gelu_from, reversed_=kn, ln=ln)
         return cuda_ops.few_rows(ln(h), weights, bias, gelu_from, reversed_=kn)
 

@@ -19,7 +19,7 @@ from ...fused_kernels_utils import ACT2FN, GELU_TANH_NAMES
 from ...modeling_utils import PretrainedConfig, PreTrainedModel
 from ...parallel.layers import Embedding, LayerNorm, Linear, RowParallelLinear
 from ...parallel.mpu import Layer, LayerPolicy
-from ..common import (AttentionCore, CausalLMHeadMixin, DecoderBackbone, SequenceClassificationMixin,
+from ..common import (AttentionCore, CausalLMHeadMixin, DecoderBackbone, SequenceClassificationMixin, foldable_norm,
                       maybe_dropout, merge_heads, to_token_rows, unhooked)
 
 
@@ -217,12 +217,9 @@ class GPTJBlock(nn.Module):
 
     def _fold_ln(self, hidden_states: Tensor) -> bool:
         """Whether ``ln_1`` of these few rows is computed inside the packed projection's kernel."""
-        from ...ops import cuda_ops
         ln = self.ln_1
-        return (hidden_states.is_cuda and type(ln) is LayerNorm and ln.oslo_fused and ln.weight is not None and unhooked(ln)
-                and cuda_ops.folded_ln_ok(hidden_states) and ln.weight.dtype == hidden_states.dtype
-                and ln.weight.numel() == hidden_states.size(-1)
-                and not (torch.is_grad_enabled() and (ln.weight.requires_grad or hidden_states.requires_grad)))
+        return (hidden_states.is_cuda and type(ln) is LayerNorm and ln.oslo_fused and unhooked(ln) and foldable_norm(ln, hidden_states)
+                and not (torch.is_grad_enabled() and hidden_states.requires_grad))
 
     def _decode_step(self, hidden_states: Tensor, packed, kw):
         """Whole block for one new token per row on a device-positioned static cache, in three launches: (LayerNorm and

@@ -242,3 +242,74 @@ def test_gptj_tensor_parallel_step_adds_the_residual_after_the_reduction(kernels
     inside = rows <= 4 and rank == 0
     for (bias, residual, y), z in zip(products, reduced):
         assert (bias is not None) == inside and (residual is not None) == inside and z is y
+
+
+def _reached(out):
+    """The leaves that a backward pass from ``out`` reaches through nodes that have one."""
+    seen, keep, stack, leaves = set(), [], [out.grad_fn], []
+    while stack:
+        node = stack.pop()
+        if node is None or id(node) in seen or "NotImplemented" in node.name():
+            continue
+        seen.add(id(node))
+        keep.append(node)
+        if hasattr(node, "variable"):
+            leaves.append(node.variable)
+        stack += [fn for fn, _ in node.next_functions]
+    return leaves
+
+
+@pytest.mark.parametrize("kind", ["gpt2", "gpt_neo", "gptj"])
+@pytest.mark.parametrize("which", ["weight", "bias"])
+def test_a_step_with_trainable_norms_keeps_their_graph(kernels, kind, which):
+    """Frozen layers, norms that learn: a step with gradients enabled is part of the graph."""
+    from oslo_b200.models.common import StaticKVCache
+    cls, cfg = _model(kind)
+    with FakeTensorMode():
+        with torch.device("cuda"):
+            model = cls._from_config(cfg, torch_dtype=torch.bfloat16)
+        model.fuse().eval().requires_grad_(False)
+        block = model.transformer.h[0]
+        x = torch.zeros(2, 1, 512, dtype=torch.bfloat16, device="cuda")
+        cache = StaticKVCache(100)
+        with torch.no_grad():
+            model(input_ids=_ids(), past_key_values=cache, use_cache=True)
+        cache.use_device_positions()
+        kw = dict(cache=cache, layer_id=0, use_cache=True, position_ids=torch.full((2, 1), 64, dtype=torch.long, device="cuda"))
+        assert not block(x, **kw)[0].requires_grad
+        norm = block.ln_1 if kind == "gptj" else block.ln_2       # the one with a way past the attention kernel, which has no backward
+        p = getattr(norm, which).requires_grad_(True)
+        assert any(leaf is p for leaf in _reached(block(x, **kw)[0]))
+
+
+@pytest.mark.parametrize("kind", ["gpt2", "gpt_neo", "gptj"])
+def test_a_step_with_a_norm_bias_of_another_type(kernels, monkeypatch, kind):
+    """No kernel takes such a bias: the norm stays a call of its own."""
+    from oslo_b200.models.common import StaticKVCache
+    from oslo_b200.ops import cuda_ops
+    folded = []
+    old = cuda_ops.few_rows
+    monkeypatch.setattr(cuda_ops, "few_rows", lambda *a, **k: folded.append(k.get("ln")) or old(*a, **k))
+    cls, cfg = _model(kind)
+    with FakeTensorMode():
+        with torch.device("cuda"):
+            model = cls._from_config(cfg, torch_dtype=torch.bfloat16)
+        model.fuse().eval().requires_grad_(False)
+        cache = StaticKVCache(100)
+        model(input_ids=_ids(), past_key_values=cache, use_cache=True)
+        cache.use_device_positions()
+        block = model.transformer.h[0]
+        kw = dict(cache=cache, layer_id=0, use_cache=True, position_ids=torch.full((2, 1), 64, dtype=torch.long, device="cuda"))
+        x = torch.zeros(2, 1, 512, dtype=torch.bfloat16, device="cuda")
+        folded.clear()
+        block(x, **kw)
+        assert any(ln is not None for ln in folded)
+        norms = [getattr(block, n) for n in ("ln_1", "ln_2") if hasattr(block, n)]
+        for ln in norms:
+            ln.bias = torch.nn.Parameter(ln.bias.float(), requires_grad=False)
+        folded.clear()
+        try:
+            block(x, **kw)
+        except RuntimeError as e:       # the norm's own call may not take it either
+            assert "LayerNorm" not in str(e)
+        assert not any(ln is not None for ln in folded)
