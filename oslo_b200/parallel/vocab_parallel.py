@@ -150,9 +150,11 @@ class _LinearCrossEntropy(torch.autograd.Function):
         on_kernels = fused and hidden.is_cuda and (ctx.in_epilogue or weight.size(0) % 8 == 0)
         dw = None if on_kernels else torch.zeros_like(weight, dtype=torch.float32)
         dw_acc = None
-        # weights whose gradient lives in the optimizer's flat buffer take the chunks' products there directly
+        # weights whose gradient lives in the optimizer's flat buffer take the chunks' products there directly, one rounding to 16
+        # bits a chunk; for a vocabulary whose size is no multiple of 8 several chunks are summed in 32 bits first and rounded once
         direct_dw = (on_kernels and getattr(weight, "_oslo_accum_grad", False) and weight.grad is not None
-                     and weight.grad.dtype == weight.dtype and weight.grad.is_contiguous() and ctx.needs_input_grad[1])
+                     and weight.grad.dtype == weight.dtype and weight.grad.is_contiguous() and ctx.needs_input_grad[1]
+                     and (n <= ctx.chunk or weight.size(0) % 8 == 0))
         db = torch.zeros(weight.size(0), dtype=torch.float32, device=weight.device) if bias is not None else None
         for s in range(0, n, ctx.chunk):
             e = min(n, s + ctx.chunk)

@@ -42,6 +42,27 @@ def test_loss_of_a_vocabulary_of_any_size(vocab, rows, with_bias, dtype):
         assert _rel(got.grad, leaf.grad) < 4 * unit, (vocab, got.shape, _rel(got.grad, leaf.grad))
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("vocab, held", [(1003, False), (1007, True)])
+def test_loss_gradient_sums_its_chunks_in_32_bits(vocab, held, dtype):
+    """Sixteen row chunks into a gradient that lives in a flat buffer. One rounding to 16 bits has an rms error of 0.42 u of the value's
+    (u = 2^-8 or 2^-11, mantissas of all kinds); the gradient matrix and the sum have one each, 0.6 u together, and an addition to a
+    gradient of the same size one more at half the weight. 0.8 u allowed; sixteen roundings of growing sums come to 1.2 u and more."""
+    ops, _ = _ops()
+    gen = torch.Generator(device="cuda").manual_seed(vocab)
+    mk = lambda *s, std: torch.randn(*s, device="cuda", generator=gen).mul_(std).to(dtype)      # noqa: E731
+    h, w = mk(512, 256, std=0.5), mk(vocab, 256, std=0.1).requires_grad_(True)
+    lab = torch.randint(0, vocab, (512,), device="cuda", generator=gen)
+    wide = w.detach().double().requires_grad_(True)
+    want, = torch.autograd.grad(torch.nn.functional.cross_entropy(h.double() @ wide.t(), lab) * 256, wide)
+    base = torch.zeros_like(w) if not held else want.to(dtype)
+    w.grad, w._oslo_accum_grad = base.detach().clone(), True
+    (ops.linear_cross_entropy(h, w, None, lab, chunk_rows=32) * 256).backward()
+    u = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+    want = want + base.double()
+    assert _rel(w.grad, want) < 0.8 * u, _rel(w.grad, want) / u
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("cols", [8, 256, 264, 512, 520, 768, 1024, 1032, 2048, 2056, 4096, 4104, 6144, 6152, 8192])
 @pytest.mark.parametrize("rows", [1, 7, 1300])
