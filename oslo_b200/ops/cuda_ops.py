@@ -80,7 +80,7 @@ def reset_device_error(like: Tensor) -> None:
 def _as_operand(t: Tensor) -> Tensor:
     """2-D tensor with contiguous last dim, 16-byte aligned rows."""
     if t.stride(-1) != 1 or t.stride(0) % 8 or t.data_ptr() % 16 or t.stride(0) < t.size(1):
-        t = t.contiguous()
+        t = t.clone(memory_format=torch.contiguous_format)     # a copy also of what is contiguous but misaligned, or one row of an odd stride
     return t
 
 
@@ -393,7 +393,7 @@ def few_rows(x: Tensor, weights, bias: Optional[Tensor] = None, gelu_from: int =
 
 def _rows_of(x: Tensor) -> Tensor:
     x = x.reshape(-1, x.size(-1))
-    return x if x.stride(1) == 1 or x.size(1) == 1 else x.contiguous()
+    return x if x.stride(1) == 1 else x.clone(memory_format=torch.contiguous_format)
 
 
 def small_m_ok(x: Tensor, *weights: Tensor) -> bool:

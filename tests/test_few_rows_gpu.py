@@ -48,6 +48,24 @@ def test_few_rows(dtype, kn, m, k1, k2, n):
         assert torch.isfinite(y).all() and (y.double() - ref).norm() <= bound
 
 
+@pytest.mark.parametrize("rows", [1, 3, 9])
+@pytest.mark.parametrize("n", [40, 37, 1])
+def test_linear_of_operands_at_odd_addresses(rows, n):
+    """Views that start between 16-byte boundaries, or single rows cut out of longer odd ones, are copied."""
+    from oslo_b200.ops import cuda_ops
+    torch.manual_seed(n)
+    buf = torch.randn(64 * 64 + 64 * 67, device="cuda").bfloat16()
+    weights = [buf[3:3 + n * 64].view(n, 64), buf[:n * 64].view(n, 64)]
+    inputs = [buf[5:5 + rows * 64].view(rows, 64), buf[:rows * 67].view(rows, 67)[:, :64], buf[8:8 + rows * 64].view(rows, 64)]
+    with torch.no_grad():
+        for w in weights:
+            for x in inputs:
+                _close(ob.ops.linear(x, w), x.double() @ w.double().t(), torch.bfloat16)
+                res = buf[:2 * rows * n:2].view(n, rows).t()
+                y = cuda_ops.linear(x, w, None, False, None, res)
+                _close(y, x.double() @ w.double().t() + res.double(), torch.bfloat16)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("d, rotary", [(8, 0), (32, 8), (64, 0), (80, 32), (128, 64), (256, 64), (256, 0)])
 @pytest.mark.parametrize("b, h, t, at, window", [(1, 3, 1, 0, 0), (2, 12, 180, 173, 0), (8, 16, 512, 300, 0), (1, 16, 2048, 2047, 0), (3, 5, 700, 690, 256),
