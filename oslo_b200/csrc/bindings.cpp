@@ -1019,7 +1019,7 @@ std::tuple<Tensor, Tensor> hyper_join(const Tensor& x, const optional<Tensor>& y
   return {xo, h};
 }
 
-// x [P, M <= 4, K] (rows of a part contiguous in K), w [P, N, K] -> [P, M, N]
+// x [P, M <= 8, K] (rows of a part contiguous in K), w [P, N, K] -> [P, M, N]
 Tensor gemv_stacked(const Tensor& x, const Tensor& w) {
   TORCH_CHECK(x.is_cuda() && x.dim() == 3 && w.dim() == 3 && x.stride(2) == 1 && w.is_contiguous() && x.size(0) == w.size(0) &&
                   x.size(2) == w.size(2) && x.scalar_type() == w.scalar_type(), "gemv_stacked: operands");

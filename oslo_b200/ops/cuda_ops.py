@@ -875,7 +875,8 @@ def stacked_linear(x: Tensor, weight: Tensor):
     n = weight.size(1)
     if not (gemm_ok(x[0], weight[0]) and n % 8 == 0):
         return torch.matmul(x, weight.transpose(1, 2)).unbind(0)
-    if rows <= STACKED_ROWS:
+    if (rows <= STACKED_ROWS and weight.is_contiguous() and x.stride(2) == 1 and not (x.stride(0) % 8 or x.stride(1) % 8)
+            and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0):
         return _ext().gemv_stacked(x, weight).unbind(0)
     if rows <= SMALL_M_ROWS and x.is_contiguous() and weight.is_contiguous():
         flat, w = x.view(parts * rows, k), weight.view(parts * n, k)

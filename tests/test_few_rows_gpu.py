@@ -66,6 +66,23 @@ def test_linear_of_operands_at_odd_addresses(rows, n):
                 _close(y, x.double() @ w.double().t() + res.double(), torch.bfloat16)
 
 
+@pytest.mark.parametrize("rows", [1, 4, 5, 8, 9])
+@pytest.mark.parametrize("layout", ["plain", "transposed weight", "sliced x", "odd x"])
+def test_stacked_products_of_any_layout(rows, layout):
+    from oslo_b200.ops import cuda_ops
+    torch.manual_seed(rows)
+    parts, k, n = 3, 64, 40
+    mk = lambda *s: torch.randn(*s, device="cuda").bfloat16()  # noqa: E731
+    w = mk(parts, k, n).transpose(1, 2) if layout == "transposed weight" else mk(parts, n, k)
+    x = mk(parts, rows, k)
+    if layout == "sliced x":
+        x = mk(parts, rows, 2 * k)[:, :, k:]
+    elif layout == "odd x":
+        x = mk(parts, rows, k + 3)[:, :, 1:k + 1]
+    for i, y in enumerate(cuda_ops.stacked_linear(x, w)):
+        _close(y, x[i].double() @ w[i].double().t(), torch.bfloat16)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("d, rotary", [(8, 0), (32, 8), (64, 0), (80, 32), (128, 64), (256, 64), (256, 0)])
 @pytest.mark.parametrize("b, h, t, at, window", [(1, 3, 1, 0, 0), (2, 12, 180, 173, 0), (8, 16, 512, 300, 0), (1, 16, 2048, 2047, 0), (3, 5, 700, 690, 256),
