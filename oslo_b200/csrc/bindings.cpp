@@ -243,17 +243,22 @@ Tensor few_rows(const Tensor& x1, const optional<Tensor>& x2, const std::vector<
   c10::cuda::CUDAGuard guard(x1.device());
   if (M > 8 && two && K1 % 64)                 // a k block of the tensor-core kernel comes from one of the inputs
     return few_rows(at::cat({x1, *x2}, 1), optional<Tensor>(), w, w_kn, bias, gelu_from, res, ln_w, ln_b, eps);
-  if (M > 8 && parts > 1 && (N / parts) % 128) // ... and a tile from one of the weights
-    return few_rows(x1, x2, {at::cat(w, 0)}, w_kn, bias, gelu_from, res, ln_w, ln_b, eps);
   Tensor y = at::empty({M, N}, x1.options());
   auto& st = dev_state(x1.get_device());
-  check_rc(oslo_few_rows(x1.data_ptr(), static_cast<int>(x1.stride(0)), static_cast<int>(K1), two ? x2->data_ptr() : nullptr,
-                         two ? static_cast<int>(x2->stride(0)) : 0, static_cast<int>(K2), w[0].data_ptr(),
-                         parts > 1 ? w[1].data_ptr() : nullptr, parts > 2 ? w[2].data_ptr() : nullptr, static_cast<int>(parts),
-                         static_cast<int>(w[0].stride(0)), static_cast<int>(w_kn), b, has_res ? res->data_ptr() : nullptr,
-                         has_res ? static_cast<int>(res->stride(0)) : 0, lw, lb, static_cast<float>(eps), y.data_ptr(),
-                         static_cast<int>(N), static_cast<int>(M), static_cast<int>(N), static_cast<int>(gelu_from), dt_code(x1),
-                         st.err.data_ptr<int>(), usable_sms(st), cur_stream()), "few_rows");
+  // ... and a tile from one of the weights: of other widths each has a launch of its own, on its columns of y
+  const int64_t launches = M > 8 && parts > 1 && (N / parts) % 128 ? parts : 1, cols = N / launches, each = parts / launches;
+  const auto at_col = [&](const void* p, int64_t c) -> const void* { return p ? static_cast<const char*>(p) + c * x1.element_size() : nullptr; };
+  for (int64_t i = 0; i < launches; ++i) {
+    const int64_t from = gelu_from < 0 ? gelu_from : std::max<int64_t>(gelu_from - i * cols, 0);
+    check_rc(oslo_few_rows(x1.data_ptr(), static_cast<int>(x1.stride(0)), static_cast<int>(K1), two ? x2->data_ptr() : nullptr,
+                           two ? static_cast<int>(x2->stride(0)) : 0, static_cast<int>(K2), w[i].data_ptr(),
+                           each > 1 ? w[1].data_ptr() : nullptr, each > 2 ? w[2].data_ptr() : nullptr, static_cast<int>(each),
+                           static_cast<int>(w[0].stride(0)), static_cast<int>(w_kn), at_col(b, i * cols),
+                           at_col(has_res ? res->data_ptr() : nullptr, i * cols), has_res ? static_cast<int>(res->stride(0)) : 0, lw, lb,
+                           static_cast<float>(eps), const_cast<void*>(at_col(y.data_ptr(), i * cols)), static_cast<int>(N),
+                           static_cast<int>(M), static_cast<int>(cols), static_cast<int>(from), dt_code(x1), st.err.data_ptr<int>(),
+                           usable_sms(st), cur_stream()), "few_rows");
+  }
   return y;
 }
 Tensor gemm_small_m(const Tensor& a, const Tensor& b, int64_t b_mn, const optional<Tensor>& bias, int64_t gelu_from) {

@@ -66,6 +66,23 @@ def test_linear_of_operands_at_odd_addresses(rows, n):
                 _close(y, x.double() @ w.double().t() + res.double(), torch.bfloat16)
 
 
+@pytest.mark.parametrize("m", [9, 64])
+@pytest.mark.parametrize("k, n", [(1024, 1032), (2048, 136)])
+def test_several_weights_of_any_width_are_not_copied(m, k, n):
+    """Widths that are no multiple of the tile's 128 columns: no memory but the result's."""
+    from oslo_b200.ops import cuda_ops
+    torch.manual_seed(n)
+    mk = lambda *s: torch.randn(*s, device="cuda").bfloat16()  # noqa: E731
+    x, ws, bias, res = mk(m, k), [mk(n, k) for _ in range(3)], mk(3 * n), mk(m, 3 * n)
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    y = cuda_ops._ext().few_rows(x, None, ws, 0, bias, n + 40, res)
+    assert torch.cuda.max_memory_allocated() - before < 2 * n * k * 2
+    z = torch.cat([x.double() @ w.double().t() for w in ws], 1) + bias.double()
+    z[:, n + 40:] = torch.nn.functional.gelu(z[:, n + 40:], approximate="tanh")
+    _close(y, z + res.double(), torch.bfloat16)
+
+
 @pytest.mark.parametrize("rows", [1, 4, 5, 8, 9])
 @pytest.mark.parametrize("layout", ["plain", "transposed weight", "sliced x", "odd x"])
 def test_stacked_products_of_any_layout(rows, layout):
