@@ -261,14 +261,28 @@ Tensor few_rows(const Tensor& x1, const optional<Tensor>& x2, const std::vector<
   }
   return y;
 }
+// The same for one weight, and up to 128 rows; any N and K whose operands have aligned rows (sizes that are no multiple of 8 are padded or
+// transposed by a copy: no layer of this package has such).
 Tensor gemm_small_m(const Tensor& a, const Tensor& b, int64_t b_mn, const optional<Tensor>& bias, int64_t gelu_from) {
-  if (a.size(0) > 64 || (b_mn && b.size(1) % 8)) {
-    TORCH_CHECK(gelu_from <= 0, "gemm_small_m: an activation on some columns needs at most 64 rows");
+  check_2d_operand(a, "a");
+  const int64_t M = a.size(0), N = b_mn ? b.size(1) : b.size(0), K = a.size(1);
+  TORCH_CHECK(b.dim() == 2 && (b_mn ? b.size(0) : b.size(1)) == K, "gemm_small_m: contraction sizes differ");
+  if (M > 64 && M <= 128 && (gelu_from > 0 || N % 8))
+    return at::cat({gemm_small_m(a.narrow(0, 0, 64), b, b_mn, bias, gelu_from), gemm_small_m(a.narrow(0, 64, M - 64), b, b_mn, bias, gelu_from)});
+  if (M > 64) {
+    TORCH_CHECK(gelu_from <= 0, "gemm_small_m: an activation on some columns needs at most 128 rows");
     const bool has_bias = bias.has_value() && bias->defined();
     const int64_t fl = (has_bias ? GEMM_FLAG_BIAS : 0) | (gelu_from == 0 ? GEMM_FLAG_GELU : 0) | (gelu_from == OSLO_ACT_RELU2 ? GEMM_FLAG_RELU2 : 0);
     return gemm(a, b, 0, b_mn, bias, optional<Tensor>(), optional<Tensor>(), optional<Tensor>(), fl, 1.0);
   }
-  return few_rows(a, optional<Tensor>(), {b}, b_mn, bias, gelu_from, optional<Tensor>(), optional<Tensor>(), optional<Tensor>(), 0.0);
+  Tensor x = a, w = b;
+  if (b_mn && N % 8) { w = w.t().contiguous(); b_mn = 0; }
+  if (K % 8) {
+    const int64_t more = 8 - K % 8;
+    x = at::constant_pad_nd(x, {0, more});
+    w = b_mn ? at::constant_pad_nd(w, {0, 0, 0, more}) : at::constant_pad_nd(w, {0, more});
+  }
+  return few_rows(x, optional<Tensor>(), {w}, b_mn, bias, gelu_from, optional<Tensor>(), optional<Tensor>(), optional<Tensor>(), 0.0);
 }
 
 // grad [V, W] += rows of dy [n, W] by ids [n]

@@ -83,6 +83,23 @@ def test_several_weights_of_any_width_are_not_copied(m, k, n):
     _close(y, z + res.double(), torch.bfloat16)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("kn", [False, True])
+@pytest.mark.parametrize("m", [64, 65, 128])
+@pytest.mark.parametrize("k, n", [(64, 72), (60, 72), (64, 68), (4104, 1000)])
+@pytest.mark.parametrize("gelu_from", [-1, 0, 24])
+def test_small_products_of_up_to_128_rows(dtype, kn, m, k, n, gelu_from):
+    """The operator on operands whose rows are aligned, whatever their sizes."""
+    from oslo_b200.ops import cuda_ops
+    torch.manual_seed(m + k + n)
+    mk = lambda r, c: torch.randn(r, -(-c // 8) * 8, device="cuda").to(dtype)[:, :c]  # noqa: E731
+    a, b, bias = mk(m, k), mk(k, n) if kn else mk(n, k), torch.randn(n, device="cuda").to(dtype)
+    z = a.double() @ (b.double() if kn else b.double().t()) + bias.double()
+    if gelu_from >= 0:
+        z[:, gelu_from:] = torch.nn.functional.gelu(z[:, gelu_from:], approximate="tanh")
+    _close(cuda_ops._ext().gemm_small_m(a, b, int(kn), bias, gelu_from), z, dtype)
+
+
 @pytest.mark.parametrize("rows", [1, 4, 5, 8, 9])
 @pytest.mark.parametrize("layout", ["plain", "transposed weight", "sliced x", "odd x"])
 def test_stacked_products_of_any_layout(rows, layout):
