@@ -290,10 +290,13 @@ void embedding_grad_(Tensor grad, const Tensor& ids, const Tensor& dy) {
   TORCH_CHECK(grad.is_cuda() && grad.dim() == 2 && grad.is_contiguous() && dy.dim() == 2 && dy.is_contiguous() && dy.size(1) == grad.size(1) &&
                   dy.scalar_type() == grad.scalar_type() && dy.device() == grad.device(), "embedding_grad: grad and dy");
   TORCH_CHECK(ids.scalar_type() == at::kLong && ids.is_contiguous() && ids.numel() == dy.size(0) && ids.device() == grad.device(), "embedding_grad: ids");
+  TORCH_CHECK(dy.size(0) <= OSLO_EMBED_GRAD_TOKENS && grad.size(1) <= INT32_MAX, "embedding_grad: at most ", OSLO_EMBED_GRAD_TOKENS, " tokens");
   c10::cuda::CUDAGuard guard(grad.device());
-  check_rc(oslo_embedding_grad(reinterpret_cast<const long long*>(ids.data_ptr<int64_t>()), dy.data_ptr(), grad.data_ptr(),
-                               static_cast<int>(dy.size(0)), grad.size(0), static_cast<int>(grad.size(1)), dt_code(grad),
-                               dev_state(grad.get_device()).err.data_ptr<int>(), cur_stream()), "embedding_grad");
+  const int n = static_cast<int>(dy.size(0)), width = static_cast<int>(grad.size(1));
+  Tensor ws = at::empty({oslo_embedding_grad_bytes(n, width)}, grad.options().dtype(at::kByte));
+  check_rc(oslo_embedding_grad(reinterpret_cast<const long long*>(ids.data_ptr<int64_t>()), dy.data_ptr(), grad.data_ptr(), ws.data_ptr(), n,
+                               grad.size(0), width, dt_code(grad), dev_state(grad.get_device()).err.data_ptr<int>(), cur_stream(3)),
+           "embedding_grad");
 }
 
 std::tuple<Tensor, Tensor, Tensor> layernorm_fwd(const Tensor& x, const Tensor& w, const optional<Tensor>& b, double eps) {

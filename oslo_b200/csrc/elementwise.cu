@@ -698,101 +698,151 @@ __global__ void __launch_bounds__(CS_WARPS * 32) ce_reduce_stats_kernel(const fl
 }
 
 // ---------------------------------------------------------------------- embedding gradient
-// grad[id] += sum of dy[t] over the tokens t with ids[t] == id, in 32 bits and in token order, rounded once. A block owns the ids of one
-// bucket and a range of columns: it lists its tokens (every block reads all ids, which fit L2 many times over), then sums the rows of
-// each id. Bound by dy and the touched rows of grad; the library's gradient sorts the ids, sums segments through workspaces, fills a
-// whole [vocabulary, width] tensor and adds that to grad (50400 x 4096, 8192 tokens: 1.3 ms).
-constexpr int EG_THREADS = 128, EG_LIST = 2048, EG_IDS = 8;
+// grad[id] += sum of dy[t] over the tokens t with ids[t] == id, in 32 bits, rounded once. Tokens are put in the order of their ids (of
+// equal ids: their own), the ordered list is cut into chunks of EG_CHUNK, and a block sums one chunk: ids that lie inside it go to grad,
+// the parts of an id that goes on over chunks go to a workspace and are added up in their order by a third kernel. How often an id comes
+// up does not matter then: pad tokens and token types fill whole batches with one or two ids. bf16, us, ids of all kinds / half of them
+// one pad id / two type ids: 8000 x 768 44 / 52 / 48, 7108 x 2048 46 / 54 / 50, 8192 x 4096 91 / 88 / 64, 32768 x 4096 419 / 468 / 429;
+// one block per id, its rows one after another, took 46 / 2659 / 1232, 51 / 6502 / 1128, 107 / 6225 / 1305, 639 / 22877 / 10468, the
+// library's sort and segment sums 280 / 275 / 246, 532 / 447 / 385, 991 / 825 / 655, 2450 / 2006 / 1359.
+struct __align__(8) EmbedToken { int id, t; };   // id -1: outside the vocabulary
+constexpr int EG_THREADS = 128, EG_CHUNK = 32, EG_AHEAD = 8;
+
+// order[rank of t] = token t. The rank is counted against all tokens, ER_LANES lanes to a token: n^2 comparisons from shared memory
+constexpr int ER_THREADS = 256, ER_LANES = 8, ER_TILE = 2048;
+__global__ void __launch_bounds__(ER_THREADS) embedding_order_kernel(const long long* __restrict__ ids, EmbedToken* __restrict__ order, int n,
+                                                                     long long vocab, int* err) {
+  __shared__ __align__(16) unsigned tile[ER_TILE];
+  auto key = [&](int t) { const long long id = ids[t]; return id >= 0 && id < vocab ? static_cast<unsigned>(id) : 0x80000000u; };   // vocab < 2^31
+  const int t = (blockIdx.x * ER_THREADS + threadIdx.x) / ER_LANES, lane = threadIdx.x % ER_LANES;
+  const unsigned mine = t < n ? key(t) : 0u;
+  const int own = t & ~3;                       // the four that t is one of
+  int rank = 0;
+  for (int base = 0; base < n; base += ER_TILE) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < ER_TILE; i += ER_THREADS) tile[i] = base + i < n ? key(base + i) : 0xffffffffu;
+    __syncthreads();
+#pragma unroll 4
+    for (int q = lane * 4; q < ER_TILE; q += ER_LANES * 4) {
+      const uint4 k = *reinterpret_cast<const uint4*>(tile + q);
+      const unsigned below = mine + (base + q < own ? 1u : 0u);   // equal ids come in the order of their tokens
+      rank += (k.x < below) + (k.y < below) + (k.z < below) + (k.w < below);
+    }
+  }
+#pragma unroll
+  for (int off = ER_LANES / 2; off > 0; off >>= 1) rank += __shfl_xor_sync(0xffffffffu, rank, off);
+  if (lane != 0 || t >= n) return;
+  for (int u = own; u < t; ++u) rank += key(u) == mine;
+  const bool in = mine != 0x80000000u;
+  if (!in) OSLO_REPORT_BOUNDS(err);             // no row to add to: skipped
+  order[rank] = EmbedToken{in ? static_cast<int>(mine) : -1, t};
+}
+
+__device__ __forceinline__ void store8f(float* p, const float (&f)[8]) {
+  reinterpret_cast<float4*>(p)[0] = make_float4(f[0], f[1], f[2], f[3]);
+  reinterpret_cast<float4*>(p)[1] = make_float4(f[4], f[5], f[6], f[7]);
+}
+// part [chunks][2][width]: of an id that came into the chunk from the one before, and of one that starts in it and goes on
 template <typename T>
-__global__ void __launch_bounds__(EG_THREADS) embedding_grad_kernel(const long long* __restrict__ ids, const T* __restrict__ dy, T* __restrict__ grad,
-                                                                    int n, long long vocab, int width, int buckets, int* err) {
-  __shared__ int list_id[EG_LIST], list_t[EG_LIST];
-  __shared__ int count[EG_THREADS / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int c = (blockIdx.y * EG_THREADS + threadIdx.x) * 8;
-  const bool live = c < width;
-  auto mine = [&](long long id) {
-    return id >= 0 && id < vocab && static_cast<int>((static_cast<unsigned>(id) * 2654435761u >> 8) % static_cast<unsigned>(buckets)) == static_cast<int>(blockIdx.x);
-  };
-  auto add = [&](float (&acc)[8], int t) {
-    float v[8];
-    load_vec(dy + static_cast<size_t>(t) * width + c, v);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] += v[i];
-  };
-  auto store = [&](int id, const float (&acc)[8]) {
-    float v[8];
-    T* g = grad + static_cast<size_t>(id) * width + c;
-    load_vec(g, v);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] += acc[i];
-    store_vec(g, v);
-  };
-  int total = 0;                                // tokens of this bucket, the same in every thread
-  for (int base = 0; base < n; base += EG_THREADS * EG_IDS) {   // EG_IDS consecutive tokens per thread
-    unsigned hit = 0;
-#pragma unroll
-    for (int u = 0; u < EG_IDS; ++u) {
-      const int t = base + threadIdx.x * EG_IDS + u;
-      const long long id = t < n ? ids[t] : -1;
-      if (t < n && (id < 0 || id >= vocab) && blockIdx.x == 0 && blockIdx.y == 0) OSLO_REPORT_BOUNDS(err);   // no row to add to: skipped
-      hit |= (mine(id) ? 1u : 0u) << u;
-    }
-    int before = __popc(hit);                   // inclusive over the warp's lanes
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const int o = __shfl_up_sync(0xffffffffu, before, off);
-      if (lane >= off) before += o;
-    }
-    __syncthreads();
-    if (lane == 31) count[warp] = before;
-    __syncthreads();
-    int at = total + before - __popc(hit);
-    for (int w = 0; w < EG_THREADS / 32; ++w) {
-      if (w < warp) at += count[w];
-      total += count[w];
-    }
-    for (; hit != 0; hit &= hit - 1, ++at) {
-      const int t = base + threadIdx.x * EG_IDS + __ffs(hit) - 1;
-      if (at < EG_LIST) { list_id[at] = static_cast<int>(ids[t]); list_t[at] = t; }
-    }
+__global__ void __launch_bounds__(EG_THREADS) embedding_sum_kernel(const EmbedToken* __restrict__ order, const T* __restrict__ dy, T* __restrict__ grad,
+                                                                   float* __restrict__ part, int n, int width) {
+  __shared__ int id_s[EG_CHUNK], t_s[EG_CHUNK];
+  __shared__ unsigned char ends_s[EG_CHUNK], starts_s[EG_CHUNK];   // the id's last token; its first one lies in this chunk
+  const int p0 = blockIdx.x * EG_CHUNK, count = min(EG_CHUNK, n - p0);
+  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
+  if (threadIdx.x < count) {
+    const int p = p0 + threadIdx.x;
+    const EmbedToken e = order[p];
+    id_s[threadIdx.x] = e.id; t_s[threadIdx.x] = e.t;
+    ends_s[threadIdx.x] = p + 1 == n || order[p + 1].id != e.id;
+    starts_s[threadIdx.x] = p0 == 0 || order[p0 - 1].id != e.id;   // in order: an id that did not end the chunk before starts in this one
   }
   __syncthreads();
-  if (total <= EG_LIST) {
-    for (int i = 0; i < total; ++i) {
-      const int id = list_id[i];
-      bool first = true;
-      for (int j = 0; j < i && first; ++j) first = list_id[j] != id;
-      if (!first || !live) continue;
-      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      for (int j = i; j < total; ++j)
-        if (list_id[j] == id) add(acc, list_t[j]);
-      store(id, acc);
+  if (c >= width) return;
+  float acc[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+  for (int j0 = 0; j0 < count; j0 += EG_AHEAD) {
+    uint4 x[EG_AHEAD], g[EG_AHEAD];             // rows of dy, and those of grad that they complete: no two of these are the same row
+#pragma unroll
+    for (int u = 0; u < EG_AHEAD; ++u) {
+      const int j = j0 + u;
+      if (j < count && id_s[j] >= 0) {
+        x[u] = *reinterpret_cast<const uint4*>(dy + static_cast<size_t>(t_s[j]) * width + c);
+        if (ends_s[j] && starts_s[j]) g[u] = *reinterpret_cast<const uint4*>(grad + static_cast<size_t>(id_s[j]) * width + c);
+      }
     }
-    return;
+#pragma unroll
+    for (int u = 0; u < EG_AHEAD; ++u) {
+      const int j = j0 + u;
+      if (j < count && id_s[j] >= 0) {
+        float v[8];
+        unpack_vec<T>(x[u], v);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i] += v[i];
+        if (ends_s[j] || j == count - 1) {
+          if (!starts_s[j]) {
+            store8f(part + (static_cast<size_t>(blockIdx.x) * 2) * width + c, acc);
+          } else if (!ends_s[j]) {
+            store8f(part + (static_cast<size_t>(blockIdx.x) * 2 + 1) * width + c, acc);
+          } else {
+            unpack_vec<T>(g[u], v);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] += acc[i];
+            store_vec(grad + static_cast<size_t>(id_s[j]) * width + c, v);
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+        }
+      }
+    }
   }
-  // more tokens than the list holds (an id that fills the batch): id by id, each over all tokens
-  long long last = -1;
+}
+
+// the block of the chunk in which an id starts that goes on adds up its parts
+template <typename T>
+__global__ void __launch_bounds__(EG_THREADS) embedding_join_kernel(const EmbedToken* __restrict__ order, const float* __restrict__ part,
+                                                                    T* __restrict__ grad, int n, int width) {
+  const int chunk = blockIdx.x, p0 = chunk * EG_CHUNK, next = p0 + EG_CHUNK;
+  if (next >= n) return;
+  const int id = order[next - 1].id;
+  if (id < 0 || order[next].id != id || (p0 > 0 && order[p0 - 1].id == id)) return;   // the same in every thread
+  int more = 0;                                 // chunks that it comes into
   while (true) {
-    __syncthreads();
-    if (threadIdx.x == 0) list_id[0] = 0x7fffffff;
-    __syncthreads();
-    for (int t = threadIdx.x; t < n; t += EG_THREADS) {
-      const long long id = ids[t];
-      if (id > last && mine(id)) atomicMin(&list_id[0], static_cast<int>(id));
-    }
-    __syncthreads();
-    const int id = list_id[0];
-    if (id == 0x7fffffff) break;
-    if (live) {
-      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-      for (int t = 0; t < n; ++t)
-        if (ids[t] == id) add(acc, t);
-      store(id, acc);
-    }
-    last = id;
+    const long long p = static_cast<long long>(chunk + 1 + more + threadIdx.x) * EG_CHUNK;
+    const int hits = __syncthreads_count(p < n && order[p].id == id);
+    more += hits;
+    if (hits < static_cast<int>(blockDim.x)) break;
   }
+  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
+  if (c >= width) return;
+  float acc[8], v[8];
+  const float* src = part + (static_cast<size_t>(chunk) * 2 + 1) * width + c;
+  auto add = [&](const float4& a, const float4& b) {
+    acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
+    acc[4] += b.x; acc[5] += b.y; acc[6] += b.z; acc[7] += b.w;
+  };
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+  add(reinterpret_cast<const float4*>(src)[0], reinterpret_cast<const float4*>(src)[1]);
+  src += width;                                 // head of the next chunk
+  for (int k0 = 0; k0 < more; k0 += EG_AHEAD) {
+    float4 a[EG_AHEAD], b[EG_AHEAD];
+#pragma unroll
+    for (int u = 0; u < EG_AHEAD; ++u)
+      if (k0 + u < more) {
+        const float4* q = reinterpret_cast<const float4*>(src + static_cast<size_t>(k0 + u) * 2 * width);
+        a[u] = q[0]; b[u] = q[1];
+      }
+#pragma unroll
+    for (int u = 0; u < EG_AHEAD; ++u)
+      if (k0 + u < more) add(a[u], b[u]);
+  }
+  T* g = grad + static_cast<size_t>(id) * width + c;
+  load_vec(g, v);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] += acc[i];
+  store_vec(g, v);
 }
 
 // ---------------------------------------------------------------------- AdamW / norms
@@ -1151,19 +1201,27 @@ extern "C" int oslo_ngram_ban(const long long* tokens, float* lprobs, int rows, 
   RET_LAST();
 }
 
-extern "C" int oslo_embedding_grad(const long long* ids, const void* dy, void* grad, int n, long long vocab, int width, int dtype,
+extern "C" long long oslo_embedding_grad_bytes(int n, int width) {
+  const long long chunks = (static_cast<long long>(n) + EG_CHUNK - 1) / EG_CHUNK;
+  return (n + 1) / 2 * 2 * static_cast<long long>(sizeof(EmbedToken)) + chunks * 2 * width * static_cast<long long>(sizeof(float));
+}
+extern "C" int oslo_embedding_grad(const long long* ids, const void* dy, void* grad, void* ws, int n, long long vocab, int width, int dtype,
                                    int* err_word, cudaStream_t st) {
   if (n <= 0 || width <= 0) return 0;
   if (n > OSLO_EMBED_GRAD_TOKENS || width % 8 || vocab > 0x7ffffffell || (reinterpret_cast<uintptr_t>(dy) & 15) ||
-      (reinterpret_cast<uintptr_t>(grad) & 15))
+      (reinterpret_cast<uintptr_t>(grad) & 15) || (reinterpret_cast<uintptr_t>(ws) & 15))
     return -1;
-  const int buckets = std::max(64, n / 16);     // about 16 tokens each
-  const dim3 grid(buckets, (width + EG_THREADS * 8 - 1) / (EG_THREADS * 8));
-  if (dtype == OSLO_DT_BF16)
-    embedding_grad_kernel<__nv_bfloat16><<<grid, EG_THREADS, 0, st>>>(ids, (const __nv_bfloat16*)dy, (__nv_bfloat16*)grad, n, vocab, width, buckets, err_word);
-  else if (dtype == OSLO_DT_FP16)
-    embedding_grad_kernel<__half><<<grid, EG_THREADS, 0, st>>>(ids, (const __half*)dy, (__half*)grad, n, vocab, width, buckets, err_word);
-  else
-    return -2;
+  if (dtype != OSLO_DT_BF16 && dtype != OSLO_DT_FP16) return -2;
+  EmbedToken* order = static_cast<EmbedToken*>(ws);
+  float* part = reinterpret_cast<float*>(order + (n + 1) / 2 * 2);
+  const int threads = std::min(EG_THREADS, (width / 8 + 31) / 32 * 32);
+  const dim3 grid((n + EG_CHUNK - 1) / EG_CHUNK, (width / 8 + threads - 1) / threads);
+  embedding_order_kernel<<<(n * ER_LANES + ER_THREADS - 1) / ER_THREADS, ER_THREADS, 0, st>>>(ids, order, n, vocab, err_word);
+#define EMBED_GRAD(T)                                                                                            \
+  { embedding_sum_kernel<T><<<grid, threads, 0, st>>>(order, (const T*)dy, (T*)grad, part, n, width);              \
+    embedding_join_kernel<T><<<grid, threads, 0, st>>>(order, part, (T*)grad, n, width); }
+  if (dtype == OSLO_DT_BF16) EMBED_GRAD(__nv_bfloat16)
+  else EMBED_GRAD(__half)
+#undef EMBED_GRAD
   RET_LAST();
 }

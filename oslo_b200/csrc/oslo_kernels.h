@@ -50,9 +50,11 @@ int oslo_ce_reduce_stats(const float* stats, float* rowmax, float* sumexp, float
                          cudaStream_t stream);
 
 // grad [vocab, width] (16-bit) += rows of dy [n, width] by id; n <= OSLO_EMBED_GRAD_TOKENS, width % 8 == 0; ids outside the vocabulary
-// are skipped
+// are skipped. ws: oslo_embedding_grad_bytes(n, width) bytes, 16-byte aligned. The tokens are ordered by n^2 comparisons, which sets
+// the limit (there 0.4 ms for rows of 4096, a third of the library's time; more tokens take the library's gradient)
 #define OSLO_EMBED_GRAD_TOKENS 32768
-int oslo_embedding_grad(const long long* ids, const void* dy, void* grad, int n, long long vocab, int width, int dtype, int* err_word,
+long long oslo_embedding_grad_bytes(int n, int width);
+int oslo_embedding_grad(const long long* ids, const void* dy, void* grad, void* ws, int n, long long vocab, int width, int dtype, int* err_word,
                         cudaStream_t stream);
 
 // LayerNorm over the last dim of [rows, cols]; mean/rstd are fp32 [rows]

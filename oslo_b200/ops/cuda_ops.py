@@ -248,7 +248,7 @@ def fused_mlp(x: Tensor, w_in: Tensor, b_in: Optional[Tensor], w_out: Tensor, b_
     return _FusedMLP.apply(x, w_in, b_in, w_out, b_out, residual, reversed_)
 
 
-EMBED_GRAD_TOKENS = 32768
+EMBED_GRAD_TOKENS = 32768     # OSLO_EMBED_GRAD_TOKENS of csrc/oslo_kernels.h, which says why
 
 
 class _Embedding(torch.autograd.Function):

@@ -136,6 +136,65 @@ def test_embedding_gradient_by_rows(n, vocab, width, same, dtype):
     assert _rel(w.grad, held.double() + want) <= eps
 
 
+def _time(call, repeats=20):
+    """Median device time of a call, us."""
+    for _ in range(3):
+        call()
+    marks = [torch.cuda.Event(enable_timing=True) for _ in range(repeats + 1)]
+    marks[0].record()
+    for mark in marks[1:]:
+        call()
+        mark.record()
+    torch.cuda.synchronize()
+    return sorted(a.elapsed_time(b) * 1e3 for a, b in zip(marks, marks[1:]))[repeats // 2]
+
+
+@pytest.mark.parametrize("n, width", [(8000, 768), (7108, 2048)])
+@pytest.mark.parametrize("kind", ["one pad id for half", "two type ids"])
+def test_embedding_gradient_of_ids_that_fill_a_batch(n, width, kind):
+    """Values at every place where an id can start and end in the ordered list, and no slower than three times a batch of all kinds of
+    ids (one block that adds up all rows of an id took fifty times that)."""
+    from oslo_b200.ops import cuda_ops as co
+    torch.manual_seed(n)
+    vocab = 50257
+    ids = torch.randint(0, vocab, (n,), device="cuda")
+    dy = torch.randn(n, width, device="cuda").bfloat16()
+    g = torch.zeros(vocab, width, device="cuda", dtype=torch.bfloat16)
+    mixed = _time(lambda: co._ext().embedding_grad_(g, ids, dy))
+    if kind == "two type ids":
+        ids = (torch.arange(n, device="cuda") % 1000 > 500).long() * 7
+    else:
+        ids[torch.rand(n, device="cuda") < 0.5] = vocab - 1
+    same = _time(lambda: co._ext().embedding_grad_(g, ids, dy))
+    assert same < 3 * mixed + 20, (same, mixed)
+    g.zero_()
+    co._ext().embedding_grad_(g, ids, dy)
+    want = torch.zeros(vocab, width, device="cuda", dtype=torch.float64).index_add_(0, ids, dy.double())
+    assert _rel(g, want) <= 2.0 ** -8
+    first = g.clone()
+    g.zero_()
+    co._ext().embedding_grad_(g, ids, dy)
+    assert torch.equal(g, first)
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 64, 65, 1000, 2049, 32768])
+def test_embedding_gradient_at_the_edges_of_its_chunks(n):
+    """Ids whose rows end, start and go on at chunks of 32 ordered tokens; ids outside the vocabulary are skipped."""
+    from oslo_b200.ops import cuda_ops as co
+    torch.manual_seed(n)
+    dy = torch.randn(n, 264, device="cuda").half()
+    for ids in (torch.zeros(n), torch.arange(n) // 32, (torch.arange(n) + 16) // 32, torch.arange(n) // 96, torch.arange(n).flip(0) // 33,
+                torch.arange(n) % 5, torch.arange(n) % 40 - 3):
+        ids = ids.long().cuda()
+        vocab = int(ids.max().clamp_min(0)) + 1 if int(ids.min()) >= 0 else 30
+        g = torch.zeros(vocab, 264, device="cuda").half()
+        co._ext().embedding_grad_(g, ids, dy)
+        ok = (ids >= 0) & (ids < vocab)
+        want = torch.zeros(vocab, 264, device="cuda", dtype=torch.float64).index_add_(0, ids[ok], dy[ok].double())
+        assert (g.double() - want).abs().max() <= 2.0 ** -11 * want.abs().max() + 1e-5 * n ** 0.5      # one rounding; 32-bit sums of up to n rows
+    co.reset_device_error(dy)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("rows", [296, 297, 1000])
 @pytest.mark.parametrize("cols, top", [(512, 1), (520, 3), (1024, 2), (2048, 3), (2056, 2), (4096, 5), (4104, 3)])
