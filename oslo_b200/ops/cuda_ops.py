@@ -263,9 +263,11 @@ class _Embedding(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         ids, weight = ctx.saved_tensors
-        g = weight.grad
-        direct = (g is not None and getattr(weight, "_oslo_accum_grad", False) and g.dtype == weight.dtype and g.shape == weight.shape
-                  and g.is_contiguous() and g.data_ptr() % 16 == 0 and not torch.is_grad_enabled()
+        if torch.is_grad_enabled():     # create_graph: the gradient is differentiated again
+            return None, torch.ops.aten.embedding_dense_backward(dy, ids, weight.size(0), -1, False)
+        g = weight.grad if getattr(weight, "_oslo_accum_grad", False) else None
+        direct = (g is not None and g.dtype == weight.dtype and g.shape == weight.shape
+                  and g.is_contiguous() and g.data_ptr() % 16 == 0 and _accumulates(ctx.next_functions[1][0])
                   # the data-parallel wrapper and hooks of the user count autograd's own calls here
                   and getattr(weight, "_oslo_grad_hook", None) is None and not weight._backward_hooks
                   and not getattr(weight, "_post_accumulate_grad_hooks", None))
@@ -276,8 +278,19 @@ class _Embedding(torch.autograd.Function):
         return None, (None if direct else g)
 
 
+def _accumulates(leaf) -> bool:
+    """Whether this backward pass adds to the leaf's ``.grad``: not ``torch.autograd.grad`` (the engine does not say for a leaf then), nor
+    ``backward(inputs=...)`` of others."""
+    try:
+        return torch._C._will_engine_execute_node(leaf)
+    except RuntimeError:
+        return False
+
+
 def embedding_ok(ids: Tensor, weight: Tensor) -> bool:
-    """Whether a lookup with a gradient takes ``_Embedding``."""
+    """Whether a lookup with a gradient takes ``_Embedding`` (which function transforms and forward-mode derivatives cannot look into)."""
+    if torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0:
+        return False
     return (torch.is_grad_enabled() and weight.requires_grad and weight.is_cuda and ids.is_cuda and ids.dtype == torch.long
             and weight.dtype in _16BIT and weight.dim() == 2 and weight.size(1) % 8 == 0 and 0 < ids.numel() <= EMBED_GRAD_TOKENS)
 

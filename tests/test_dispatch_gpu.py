@@ -195,6 +195,37 @@ def test_embedding_gradient_at_the_edges_of_its_chunks(n):
     co.reset_device_error(dy)
 
 
+def test_embedding_gradient_by_every_way_of_asking():
+    """``torch.autograd.grad``, ``backward(inputs=...)``, second derivatives, function transforms and forward mode, of a weight whose
+    gradient lives in a flat buffer: what the library's lookup gives (sums of a few 16-bit values; exact in 32 bits, rounded once)."""
+    from oslo_b200.parallel.layers import Embedding
+    torch.manual_seed(0)
+    ids, other = torch.randint(0, 50, (4, 33), device="cuda"), torch.randn(64, device="cuda").bfloat16().requires_grad_()
+    emb = Embedding(50, 64).to("cuda", torch.bfloat16)
+    emb.oslo_fused = True
+    w = emb.weight
+    w.grad, w._oslo_accum_grad = torch.ones_like(w), True
+    plain = torch.nn.functional.embedding
+    loss = lambda x: (x.float() * other.float()).square().sum()        # noqa: E731
+    want, = torch.autograd.grad(loss(plain(ids, w)), w)
+    got, = torch.autograd.grad(loss(emb(ids)), w)
+    assert _rel(got, want) <= 2.0 ** -8 and torch.equal(w.grad, torch.ones_like(w))
+    loss(emb(ids)).backward(inputs=[other])
+    assert torch.equal(w.grad, torch.ones_like(w))
+    second = []
+    for look in (lambda: emb(ids), lambda: plain(ids, w)):
+        g, = torch.autograd.grad(loss(look()), w, create_graph=True)
+        second.append(torch.autograd.grad(g.float().square().sum(), other)[0])
+    assert _rel(*second) <= 2.0 ** -7
+    got = torch.func.grad(lambda p: loss(torch.func.functional_call(emb, {"weight": p}, (ids,))))(w)
+    assert _rel(got, want) <= 2.0 ** -8
+    assert torch.equal(torch.func.vmap(emb)(ids), plain(ids, w))
+    with torch.autograd.forward_ad.dual_level():
+        dual = torch.autograd.forward_ad.make_dual(w.detach().requires_grad_(), torch.ones_like(w))
+        tangent = torch.autograd.forward_ad.unpack_dual(torch.func.functional_call(emb, {"weight": dual}, (ids,))).tangent
+    assert torch.equal(tangent, torch.ones_like(tangent))
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("rows", [296, 297, 1000])
 @pytest.mark.parametrize("cols, top", [(512, 1), (520, 3), (1024, 2), (2048, 3), (2056, 2), (4096, 5), (4104, 3)])
