@@ -489,30 +489,25 @@ struct ClampedUnit {
   }
 };
 
-// y = unit(gate, up) on [rows, cols] slices with row strides. A thread keeps its columns and walks the rows, ROWS of them in flight: one
-// 64-bit division per four values and one row at a time held it at 3.9 TB/s (8192 x 5440 bf16: 69 us, 63 so).
+// y = unit(gate, up) on [rows, cols] slices with row strides. Bound by memory, the same at all widths: 44.6 M values in rows of 8 to 5440
+// columns, bf16: 59.5 us, 4.49 TB/s. (Threads that keep their columns and walk the rows: 58 us at 5440 and 54 at 2048 columns, but 66 at
+// 1344, 88 at 640 and 483 at 64; with several rows side by side in a block 56 to 58 up to 640, but 70 at 1344 and 2056.)
 template <typename T, int VEC, typename Unit>
 __global__ void __launch_bounds__(256) gated_unit_kernel(const T* __restrict__ gate, long long ldg, const T* __restrict__ up,
                                                          long long ldu, T* __restrict__ out, long long rows, int cols,
                                                          const Unit unit) {
-  constexpr int ROWS = 2;
-  const int c = (blockIdx.x * 256 + threadIdx.x) * VEC;
-  if (c >= cols) return;
-  for (long long r0 = static_cast<long long>(blockIdx.y) * ROWS; r0 < rows; r0 += static_cast<long long>(gridDim.y) * ROWS) {
-    float a[ROWS][VEC], b[ROWS][VEC];
+  const long long per_row = cols / VEC;
+  const long long total = rows * per_row;
+  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
+       i += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const long long r = i / per_row;
+    const int c = static_cast<int>(i - r * per_row) * VEC;
+    float a[VEC], b[VEC];
+    load_vec<T, VEC>(gate + r * ldg + c, a);
+    load_vec<T, VEC>(up + r * ldu + c, b);
 #pragma unroll
-    for (int u = 0; u < ROWS; ++u)
-      if (r0 + u < rows) {
-        load_vec<T, VEC>(gate + (r0 + u) * ldg + c, a[u]);
-        load_vec<T, VEC>(up + (r0 + u) * ldu + c, b[u]);
-      }
-#pragma unroll
-    for (int u = 0; u < ROWS; ++u)
-      if (r0 + u < rows) {
-#pragma unroll
-        for (int k = 0; k < VEC; ++k) a[u][k] = unit(a[u][k], b[u][k]);
-        store_vec<T, VEC>(out + (r0 + u) * cols + c, a[u]);
-      }
+    for (int k = 0; k < VEC; ++k) a[k] = unit(a[k], b[k]);
+    store_vec<T, VEC>(out + r * cols + c, a);
   }
 }
 
@@ -521,22 +516,16 @@ static int gated_unit(const void* gate, long long ldg, const void* up, long long
                       const Unit& unit, int dtype, cudaStream_t stream) {
   if (rows <= 0 || cols <= 0) return 0;
   const size_t te = dtype == OSLO_DT_FP32 ? 4 : 2;
-  const auto fits = [&](int v) {
-    return cols % v == 0 && ldg % v == 0 && ldu % v == 0 && aligned_to(gate, v * te) && aligned_to(up, v * te) && aligned_to(out, v * te);
-  };
-#define GATED_UNIT(V)                                                                                                            \
-  {                                                                                                                              \
-    const int across = (cols / V + 255) / 256;                                                                                   \
-    const long long down = std::min<long long>((rows + 1) / 2, std::max(1, 148 * 16 / across));                                  \
-    gated_unit_kernel<T, V, Unit><<<dim3(across, static_cast<unsigned>(down)), 256, 0, stream>>>(                                \
-        static_cast<const T*>(gate), ldg, static_cast<const T*>(up), ldu, static_cast<T*>(out), rows, cols, unit);               \
-  }
+  const bool vec = cols % 4 == 0 && ldg % 4 == 0 && ldu % 4 == 0 && aligned_to(gate, 4 * te) && aligned_to(up, 4 * te) &&
+                   aligned_to(out, 4 * te);
+  const long long work = rows * (vec ? cols / 4 : cols);
+  const unsigned blocks = static_cast<unsigned>(std::min<long long>((work + 255) / 256, 148 * 16));
   OSLO_DISPATCH_T(dtype, {
-    if (sizeof(T) == 2 && fits(8)) GATED_UNIT(8)
-    else if (fits(4)) GATED_UNIT(4)
-    else GATED_UNIT(1)
+    if (vec) gated_unit_kernel<T, 4, Unit><<<blocks, 256, 0, stream>>>(static_cast<const T*>(gate), ldg, static_cast<const T*>(up),
+                                                                       ldu, static_cast<T*>(out), rows, cols, unit);
+    else gated_unit_kernel<T, 1, Unit><<<blocks, 256, 0, stream>>>(static_cast<const T*>(gate), ldg, static_cast<const T*>(up), ldu,
+                                                                   static_cast<T*>(out), rows, cols, unit);
   });
-#undef GATED_UNIT
   return static_cast<int>(cudaGetLastError());
 }
 

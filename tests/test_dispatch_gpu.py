@@ -195,6 +195,19 @@ def test_embedding_gradient_at_the_edges_of_its_chunks(n):
     co.reset_device_error(dy)
 
 
+@pytest.mark.parametrize("cols", [8, 64, 640, 1344, 2056])
+def test_gated_units_of_narrow_rows(cols):
+    """The same number of values in rows of any width: all of a block's threads have work (one row per block of 256 threads left 248 of
+    them idle at 64 columns)."""
+    from oslo_b200.ops import cuda_ops as co
+    from oslo_b200.ops import reference as ref
+    rows = 8192 * 5120 // cols
+    mk = lambda r, c: torch.randn(r, c, device="cuda").bfloat16()        # noqa: E731
+    a, b, wa, wb = mk(rows, cols), mk(rows, cols), mk(8192, 5120), mk(8192, 5120)
+    assert _time(lambda: co.silu_mul(a, b)) < 1.6 * _time(lambda: co.silu_mul(wa, wb)) + 10
+    assert _rel(co.silu_mul(a[:999], b[:999]), ref.silu_mul(a[:999].double(), b[:999].double())) <= 2.0 ** -8
+
+
 def test_embedding_gradient_by_every_way_of_asking():
     """``torch.autograd.grad``, ``backward(inputs=...)``, second derivatives, function transforms and forward mode, of a weight whose
     gradient lives in a flat buffer: what the library's lookup gives (sums of a few 16-bit values; exact in 32 bits, rounded once)."""
