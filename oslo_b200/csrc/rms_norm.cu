@@ -313,29 +313,28 @@ __global__ void __launch_bounds__(THREADS) branch_join_kernel(const BranchParams
   }
 }
 
-// The same for many rows of 16-bit branches without a convolution: a thread holds K chunks of eight columns of the whole row, all loads
+// The same for many rows of 16-bit branches without a convolution: a thread holds eight columns of the row, all loads
 // of the row are on their way before the first is used, and nothing is read again (above, a branch with a norm is read twice, the row
 // goes through shared memory, and the loads of a chunk wait for the chunk before):
-// 8192 x 2048 bf16 89 -> 62 us, 6000 x 2048 with three gathered rows 74 -> 52 us (three blocks per SM: 73 and 60).
-template <typename T, int K>
-__global__ void __launch_bounds__(256, K == 1 ? 4 : 2) branch_join_rows_kernel(const BranchParams p) {
+// 8192 x 2048 bf16 89 -> 62 us, 6000 x 2048 with three gathered rows 74 -> 52 us (three blocks per SM: 73 and 60). Rows of more than 2048
+// columns, two chunks a thread, lost (8192 x 3072, two branches: 148 us against 117) and stay with the kernel above.
+template <typename T>
+__global__ void __launch_bounds__(256, 4) branch_join_rows_kernel(const BranchParams p) {
   __shared__ float red[32];
   const long long row = blockIdx.x;
-  const int step = blockDim.x * 8, c0 = threadIdx.x * 8;
-  float v[K][8], y[3][K][8];
+  const int c = threadIdx.x * 8;
+  const bool in = c < p.cols;
+  float v[8], y[3][8];
+  if (in) {
+    load_vec<float, 4>(p.x + row * p.cols + c, reinterpret_cast<float (&)[4]>(v[0]));
+    load_vec<float, 4>(p.x + row * p.cols + c + 4, reinterpret_cast<float (&)[4]>(v[4]));
+  }
 #pragma unroll
-  for (int k = 0; k < K; ++k) {
-    const int c = c0 + k * step;
-    const bool in = c < p.cols;
-    if (in) load_vec<float, 4>(p.x + row * p.cols + c, reinterpret_cast<float (&)[4]>(v[k][0]));
-    if (in) load_vec<float, 4>(p.x + row * p.cols + c + 4, reinterpret_cast<float (&)[4]>(v[k][4]));
+  for (int b = 0; b < 3; ++b)
+    if (b < p.n && in) load_branch<T, 8>(p, b, row, c, y[b]);
+  if (!in) {
 #pragma unroll
-    for (int b = 0; b < 3; ++b)
-      if (b < p.n && in) load_branch<T, 8>(p, b, row, c, y[b][k]);
-    if (!in) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) v[k][i] = y[0][k][i] = y[1][k][i] = y[2][k][i] = 0.f;
-    }
+    for (int i = 0; i < 8; ++i) v[i] = y[0][i] = y[1][i] = y[2][i] = 0.f;
   }
 #pragma unroll
   for (int b = 0; b < 3; ++b) {
@@ -344,56 +343,43 @@ __global__ void __launch_bounds__(256, K == 1 ? 4 : 2) branch_join_rows_kernel(c
     if (p.w[b] != nullptr && p.normed[b]) {                // uniform over the block
       float ss = 0.f;
 #pragma unroll
-      for (int k = 0; k < K; ++k)
-#pragma unroll
-        for (int i = 0; i < 8; ++i) ss = fmaf(y[b][k][i], y[b][k][i], ss);
+      for (int i = 0; i < 8; ++i) ss = fmaf(y[b][i], y[b][i], ss);
       ss = block_sum(ss, red);
       f *= 1.0f / sqrtf(ss / p.cols + p.eps);
     }
+    if (!in) continue;
+    if (p.w[b] != nullptr) {
+      float w[8];
+      load_vec<T, 8>(static_cast<const T*>(p.w[b]) + c, w);
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int c = c0 + k * step;
-      if (c >= p.cols) continue;
-      if (p.w[b] != nullptr) {
-        float w[8];
-        load_vec<T, 8>(static_cast<const T*>(p.w[b]) + c, w);
+      for (int i = 0; i < 8; ++i) v[i] = fmaf(f * y[b][i], w[i], v[i]);
+    } else {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[k][i] = fmaf(f * y[b][k][i], w[i], v[k][i]);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v[k][i] = fmaf(f, y[b][k][i], v[k][i]);
-      }
+      for (int i = 0; i < 8; ++i) v[i] = fmaf(f, y[b][i], v[i]);
     }
   }
   float sx = 0.f;
+  if (in) {
+    store_vec<float, 4>(p.x_out + row * p.cols + c, reinterpret_cast<const float (&)[4]>(v[0]));
+    store_vec<float, 4>(p.x_out + row * p.cols + c + 4, reinterpret_cast<const float (&)[4]>(v[4]));
+    if (p.copy) store_vec<T, 8>(static_cast<T*>(p.h1) + row * p.cols + c, v);
 #pragma unroll
-  for (int k = 0; k < K; ++k) {
-    const int c = c0 + k * step;
-    if (c >= p.cols) continue;
-    store_vec<float, 4>(p.x_out + row * p.cols + c, reinterpret_cast<const float (&)[4]>(v[k][0]));
-    store_vec<float, 4>(p.x_out + row * p.cols + c + 4, reinterpret_cast<const float (&)[4]>(v[k][4]));
-    if (p.copy) store_vec<T, 8>(static_cast<T*>(p.h1) + row * p.cols + c, v[k]);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) sx = fmaf(v[k][i], v[k][i], sx);
+    for (int i = 0; i < 8; ++i) sx = fmaf(v[i], v[i], sx);
   }
   if (p.w1 == nullptr) return;
   sx = block_sum(sx, red);
+  if (!in) return;
   const float rn = 1.0f / sqrtf(sx / p.cols + p.eps);
+  float w[8], h[8];
+  load_weight<T, 8>(p.w1, p.one1, c, w);
 #pragma unroll
-  for (int k = 0; k < K; ++k) {
-    const int c = c0 + k * step;
-    if (c >= p.cols) continue;
-    float w[8], h[8];
-    load_weight<T, 8>(p.w1, p.one1, c, w);
+  for (int i = 0; i < 8; ++i) h[i] = v[i] * rn * w[i];
+  store_vec<T, 8>(static_cast<T*>(p.h1) + row * p.cols + c, h);
+  if (p.w2 != nullptr) {
+    load_weight<T, 8>(p.w2, p.one2, c, w);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) h[i] = v[k][i] * rn * w[i];
-    store_vec<T, 8>(static_cast<T*>(p.h1) + row * p.cols + c, h);
-    if (p.w2 != nullptr) {
-      load_weight<T, 8>(p.w2, p.one2, c, w);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) h[i] = v[k][i] * rn * w[i];
-      store_vec<T, 8>(static_cast<T*>(p.h2) + row * p.cols + c, h);
-    }
+    for (int i = 0; i < 8; ++i) h[i] = v[i] * rn * w[i];
+    store_vec<T, 8>(static_cast<T*>(p.h2) + row * p.cols + c, h);
   }
 }
 
@@ -612,17 +598,14 @@ extern "C" int oslo_branch_join(const OsloBranchJoin* a, long long rows, int col
   if (smem > 200 * 1024) return -3;
   const int threads = cols >= 1024 ? 256 : (cols >= 512 ? 128 : 64);
   const bool few = rows <= 296 && cols > 1024;         // at most two blocks per SM
-  bool wide = !few && te == 2 && vec && cols % 8 == 0 && cols >= 512 && cols <= 4096 && a->conv_w == nullptr && rows > 296;
+  bool wide = !few && te == 2 && vec && cols % 8 == 0 && cols >= 512 && cols <= 2048 && a->conv_w == nullptr && rows > 296;
   for (const void* t : {static_cast<const void*>(a->h1), static_cast<const void*>(a->h2), a->one1 ? nullptr : a->w1, a->one2 ? nullptr : a->w2})
     wide = wide && aligned_to(t, 16);
   for (int i = 0; i < p.n; ++i) wide = wide && p.ldy[i] % 8 == 0 && aligned_to(p.y[i], 16) && aligned_to(p.w[i], 16);
   if (wide) {
-    const int per = cols > 2048 ? 2 : 1, rows_threads = ((cols / 8 + per - 1) / per + 31) / 32 * 32;
-#define BRANCH_ROWS(T)                                                                                                           \
-    if (per == 1) branch_join_rows_kernel<T, 1><<<static_cast<unsigned>(rows), rows_threads, 0, stream>>>(p);                    \
-    else branch_join_rows_kernel<T, 2><<<static_cast<unsigned>(rows), rows_threads, 0, stream>>>(p);
-    if (dtype == OSLO_DT_BF16) { BRANCH_ROWS(__nv_bfloat16) } else { BRANCH_ROWS(__half) }
-#undef BRANCH_ROWS
+    const int rows_threads = (cols / 8 + 31) / 32 * 32;
+    if (dtype == OSLO_DT_BF16) branch_join_rows_kernel<__nv_bfloat16><<<static_cast<unsigned>(rows), rows_threads, 0, stream>>>(p);
+    else branch_join_rows_kernel<__half><<<static_cast<unsigned>(rows), rows_threads, 0, stream>>>(p);
     return static_cast<int>(cudaGetLastError());
   }
 #define BRANCH_GO(V, N, THREADS)                                                                                 \
