@@ -145,9 +145,10 @@ static bool pair_enabled() {
 
 // Into how many ranges of k the tiles of a pair GEMM's last, incomplete wave are cut (1: none). With R tiles on P pairs, ranges of 1/s
 // of k take ceil(R s / P) / s of a wave. A k block of a wave takes about 0.4 us; the second
-// kernel and the ranges' own pipeline fills cost about 8 us and a range 0.1 us for its 256 KB there and back. bf16, uncut and cut:
-// 3062 x 2048, k = 8192: 94.5 and 83.7 us; 7108 x 2048, k = 8192: 251 and 215; 768 x 768, k = 8000: 57.8 and 29.1; 4096 x 768,
-// k = 50264: 291 and 240; where the rule says no, 7108 x 2048, k = 2048: 80.3 and 82.3 (cut in four).
+// kernel and the ranges' own pipeline fills cost about 8 us and a range 0.1 us for its 256 KB there and back. bf16, operands not in L2,
+// cut and, on the tiles that are dispatched without the cut, uncut: 3062 x 2048, k = 8192: 87.0 and 100.4 us; 7108 x 2048, k = 8192: 167
+// and 197; 768 x 768, k = 8000: 27.6 and 47.1 (128 x 128 tiles); 4096 x 768, k = 50264: 263 and 315, both operands MN-major 220 and 268
+// (single CTAs' tiles 459 and 317). 7108 x 2048, k = 2048 stays whole: 61.4.
 static int pair_split(int M, int N, int K, int num_sms) {
   const int P = num_sms / 2, kblocks = (K + BK - 1) / BK;
   const long long tiles = static_cast<long long>((M + PAIR_TILE - 1) / PAIR_TILE) * ((N + PAIR_TILE - 1) / PAIR_TILE);
@@ -229,14 +230,16 @@ static int dispatch_gemm(const void* A, const void* B, int lda, int ldb, GemmPar
   const bool fp16 = (flags & GEMM_FLAG_FP16) != 0;
   // narrow outputs use the 128-wide tile so that more CTAs share the work
   const bool wide = (N >= 256) && (static_cast<long long>((M + BM - 1) / BM) * ((N + 255) / 256) >= num_sms / 2);
-  // large outputs: 256 x 256 tiles on CTA pairs. They pull a third to a half less operand data out of L2 per FLOP and win with half of
-  // the pairs idle (bf16, k = 7108, 2048 x 2048, 64 tiles: 55.8 us, 63.4 on 128 x 256 and 90.4 on 128 x 128 tiles; k = 50264,
-  // 4096 x 768, 48 tiles: 264, 298, 461), not with more (k = 8000, 768 x 3072, 36 tiles: 53.9, 60.0, 49.5), except where the idle ones
-  // take ranges of k
+  // large outputs: 256 x 256 tiles on CTA pairs. They pull a third to a half less operand data out of L2 per FLOP. Where they leave up to
+  // half of the pairs idle they win by k and by layout (bf16, weights not in L2, pairs and single CTAs' 128 x 256 or 128 x 128 tiles, as
+  // dispatched, at 2048 x 2048, 64 tiles: both operands K-major, k = 1024 13.9 and 13.8 us, 4096 30.5 and 31.8, 8192 54.5 and 58.0; with
+  // both in L2 7 % behind up to k = 4096, 54.1 and 56.9 at 8192; one MN-major, k = 512 11.0 and 10.9, 2048 19.5 and 20.3, 8192 54.5 and
+  // 57.4; both MN-major, 512 11.1 and 11.1, 2048 19.7 and 21.2, 8192 54.9 and 60.3), and where the idle ones take ranges of k
   const long long pair_tiles = static_cast<long long>((M + PAIR_TILE - 1) / PAIR_TILE) * ((N + PAIR_TILE - 1) / PAIR_TILE);
   p.split = oslo_gemm_split_ranges(M, N, K, num_sms, split_floats);
   p.split_from = static_cast<int>(pair_tiles - pair_tiles % (num_sms / 2));
-  const bool pair = pair_enabled() && M >= PAIR_TILE && N >= PAIR_TILE && (pair_tiles >= num_sms / 4 + 1 || p.split > 1);
+  const bool pair = pair_enabled() && M >= PAIR_TILE && N >= PAIR_TILE &&
+                    (pair_tiles >= num_sms / 2 || p.split > 1 || (pair_tiles >= num_sms / 4 + 1 && K >= (a_mn_major || b_mn_major ? 1024 : 4096)));
   const int bn = pair ? BM : (wide ? 256 : 128);   // B box rows: a pair's CTA stages 128 of the 256 tile columns
   CUtensorMap ta, tb;
   int rc;
