@@ -986,9 +986,13 @@ extern "C" int oslo_layernorm_fwd(const void* x, const void* w, const void* b, v
                                   int rows, int cols, float eps, int dtype, cudaStream_t st) {
   if (rows <= 0) return 0;
   DISPATCH_16(dtype, T, {
-    if (cols % VecOf<T>::N) return -3;
-    const int nvec = cols / VecOf<T>::N;
-    if (nvec > LN_THREADS * LN_MAXV) {      // wider than the registers of a block hold
+    constexpr int V = VecOf<T>::N;
+    if (cols % V) return -3;
+    const int nvec = cols / V;
+    // wider than the registers of a block hold, or many rows with four vectors of eight values per lane, which leave room for too few
+    // blocks (bf16, rows in registers and a block per row: 8192 x 8192 73.4 and 55.7 us, 700 x 8192 7.7 and 6.6, 500 x 8192 4.8 and 5.4;
+    // 32-bit values 3000 x 4096 15.6 and 19.3)
+    if (nvec > LN_THREADS * LN_MAXV || (V == 8 && nvec > 768 && rows > 592)) {
       layernorm_fwd_kernel<T><<<rows, LN_THREADS, 0, st>>>((const T*)x, (const T*)w, (const T*)b, (T*)y, mean, rstd,
                                                            rows, cols, eps);
     } else {
