@@ -333,6 +333,101 @@ __global__ void __launch_bounds__(FR_WARPS * 32, 2) few_rows_kernel(const FewRow
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
+// One row and [N, K] weights: four columns per block of 256 threads over the whole range of k, in 32-bit FMAs, with 2 x 4 weight loads of
+// 16 bytes per lane on their way. No sums meet but a block's, which is what few outputs gain from, and weights of 64 M values and more
+// stream faster (one_row_better has the line).
+constexpr int OR_THREADS = 256, OR_COLS = 4;
+__device__ __forceinline__ uint4 ld_stream_16(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+template <typename T>
+__device__ __forceinline__ void one_row_segment(const T* __restrict__ x, int K, const T* __restrict__ w, int ldw, float (&acc)[OR_COLS]) {
+  constexpr int STEP = OR_THREADS * 8;
+  for (int k = threadIdx.x * 8; k < K; k += 2 * STEP) {
+    const bool second = k + STEP < K;
+    uint4 wv[2][OR_COLS];
+#pragma unroll
+    for (int c = 0; c < OR_COLS; ++c) {
+      wv[0][c] = ld_stream_16(w + static_cast<size_t>(c) * ldw + k);
+      wv[1][c] = second ? ld_stream_16(w + static_cast<size_t>(c) * ldw + k + STEP) : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (u == 1 && !second) break;
+      const uint4 xv = *reinterpret_cast<const uint4*>(x + k + u * STEP);
+      const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w};
+#pragma unroll
+      for (int c = 0; c < OR_COLS; ++c) {
+        const uint32_t ww[4] = {wv[u][c].x, wv[u][c].y, wv[u][c].z, wv[u][c].w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 a = Few<T>::to2(xw[j]), b = Few<T>::to2(ww[j]);
+          acc[c] = fmaf(a.x, b.x, acc[c]);
+          acc[c] = fmaf(a.y, b.y, acc[c]);
+        }
+      }
+    }
+  }
+}
+template <typename T>
+__global__ void __launch_bounds__(OR_THREADS) one_row_kernel(const FewRows p) {
+  __shared__ float red[OR_THREADS / 32][OR_COLS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const T* x1 = reinterpret_cast<const T*>(p.x1) + blockIdx.y * p.sx;
+  const T* W = reinterpret_cast<const T*>(p.w[0]) + blockIdx.y * p.sw;
+  T* out = reinterpret_cast<T*>(p.out) + blockIdx.y * p.so;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  // the next kernel's blocks only where these leave room: blocks that walk several groups of columns fill the SMs to the end
+  if (p.N <= OR_COLS * gridDim.x) asm volatile("griddepcontrol.launch_dependents;");
+  for (int n0 = blockIdx.x * OR_COLS; n0 < p.N; n0 += gridDim.x * OR_COLS) {     // N % OR_COLS == 0
+    float acc[OR_COLS] = {0.f, 0.f, 0.f, 0.f};
+    const T* w = W + static_cast<size_t>(n0) * p.ldw;
+    one_row_segment<T>(x1, p.K1, w, p.ldw, acc);
+    if (p.x2 != nullptr) one_row_segment<T>(reinterpret_cast<const T*>(p.x2), p.K - p.K1, w + p.K1, p.ldw, acc);
+#pragma unroll
+    for (int c = 0; c < OR_COLS; ++c) {
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], off);
+      if (lane == 0) red[warp][c] = acc[c];
+    }
+    __syncthreads();
+    if (threadIdx.x < OR_COLS) {
+      const int n = n0 + threadIdx.x;
+      float v = 0.f;
+#pragma unroll
+      for (int i = 0; i < OR_THREADS / 32; ++i) v += red[i][threadIdx.x];
+      if (p.bias) v += Few<T>::to(reinterpret_cast<const T*>(p.bias)[n]);
+      if (p.gelu_from >= 0 && n >= p.gelu_from) v = few_gelu(v);
+      if (p.gelu_from == OSLO_ACT_RELU2) { v = fmaxf(v, 0.f); v *= v; }
+      if (p.res) v += Few<T>::to(reinterpret_cast<const T*>(p.res)[n]);
+      out[n] = Few<T>::from(v);
+    }
+    __syncthreads();
+  }
+}
+// Columns of all products that one wave of blocks covers, or weights large enough to be bound by bandwidth alone (bf16, cold weights, us,
+// one_row_kernel and few_rows_kernel: [768, 768] 2.4 and 2.9, [2304, 768] 3.0 and 3.5, [2048, 8192] 7.7 and 7.9, [4096, 20480] 28.2 and 31.9,
+// [50400, 4096] 63.5 and 69.6; in between [3072, 768] 4.4 and 3.7, [4096, 4096] 8.7 and 7.9, [8192, 2048] 9.1 and 7.1)
+static bool one_row_better(const FewRows& p, int stacked, int num_sms) {
+  const long long cols = static_cast<long long>(p.N) * stacked;
+  return p.M == 1 && p.N % OR_COLS == 0 && (cols <= 4ll * OR_COLS * num_sms || cols * p.K >= 64ll << 20);
+}
+template <typename T>
+static int one_row_launch(const FewRows& p, int stacked, int num_sms, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(std::max(1, std::min(p.N / OR_COLS, 8 * num_sms / stacked))), stacked);
+  cfg.blockDim = dim3(OR_THREADS);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, one_row_kernel<T>, p));
+}
+
 template <typename T, bool KN, bool LN>
 static int few_launch(FewRows& p, int stacked, int num_sms, cudaStream_t st) {
   using S = FewShape<KN, LN>;
@@ -363,6 +458,7 @@ static int few_launch(FewRows& p, int stacked, int num_sms, cudaStream_t st) {
 template <typename T>
 static int few_dispatch(FewRows& p, bool kn, int parts, int num_sms, cudaStream_t st) {
   const bool ln = p.ln_w != nullptr;
+  if (!kn && !ln && p.Np == p.N && one_row_better(p, parts, num_sms)) return one_row_launch<T>(p, parts, num_sms, st);
   if (kn) return ln ? few_launch<T, true, true>(p, parts, num_sms, st) : few_launch<T, true, false>(p, parts, num_sms, st);
   return ln ? few_launch<T, false, true>(p, parts, num_sms, st) : few_launch<T, false, false>(p, parts, num_sms, st);
 }
