@@ -696,7 +696,10 @@ extern "C" int oslo_few_rows(const void* x1, int ld1, int K1, const void* x2, in
   p.bias = bias; p.res = res; p.ln_w = ln_w; p.ln_b = ln_b; p.out = out; p.eps = eps;
   p.ld1 = ld1; p.ld2 = ld2; p.ldw = ldw; p.ldr = ldr; p.ldo = ldo; p.M = M; p.N = N; p.Np = N / parts;
   p.K1 = K1; p.K = K1 + K2; p.gelu_from = gelu_from;
-  const bool kn = w_kn != 0, tc = M > FR_ROWS;
+  // [K, N] weights of more than 6 M values stream through the tensor cores whatever the rows: few_rows_kernel's transposed fragments hold
+  // them at 3 TB/s ([4096, 28672], 1 and 8 rows: 77.8 and 79.9 us, 41.0 and 42.0 so; [768, 3072]: 4.3 and 4.8, 5.6)
+  const bool kn = w_kn != 0;
+  const bool tc = M > FR_ROWS || (kn && !ln_w && static_cast<long long>(p.K) * N > 6ll << 20 && (!x2 || K1 % FT_BK == 0));
   if (dtype == OSLO_DT_BF16)
     return tc ? few_tc_dispatch<__nv_bfloat16>(p, kn, parts, err_word, num_sms, stream) : few_dispatch<__nv_bfloat16>(p, kn, 1, num_sms, stream);
   if (dtype == OSLO_DT_FP16)

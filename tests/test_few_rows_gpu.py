@@ -48,6 +48,22 @@ def test_few_rows(dtype, kn, m, k1, k2, n):
         assert torch.isfinite(y).all() and (y.double() - ref).norm() <= bound
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("kn, m, k1, k2, n", [(0, 1, 8200, 8184, 4100), (0, 1, 16384, 0, 4098), (0, 1, 2056, 0, 2368), (0, 1, 2048, 8, 2372), (0, 2, 16392, 0, 4100),
+                                              (1, 1, 4104, 0, 2048), (1, 8, 4096, 8, 2056), (1, 3, 4088, 16, 2048), (1, 5, 3072, 0, 2048), (1, 5, 3080, 0, 2048)])
+def test_few_rows_on_both_sides_of_the_rules_for_large_weights(dtype, kn, m, k1, k2, n):
+    """One row with few outputs or 64 M values and more; [in, out] weights below and above 6 M values, their k from one and two inputs."""
+    from oslo_b200.ops import cuda_ops
+    torch.manual_seed(k1 + n)
+    mk = lambda *s: torch.randn(*s, device="cuda").to(dtype)  # noqa: E731
+    x1, x2, bias, res = mk(m, k1), (mk(m, k2) if k2 else None), mk(n), mk(m, n)
+    w = mk(k1 + k2, n) if kn else mk(n, k1 + k2)
+    x = x1 if x2 is None else torch.cat([x1, x2], 1)
+    z = x.double() @ (w.double() if kn else w.double().t()) + bias.double()
+    z[:, n // 2:] = torch.nn.functional.gelu(z[:, n // 2:], approximate="tanh")
+    _close(cuda_ops._ext().few_rows(x1, x2, [w], kn, bias, n // 2, res), z + res.double(), dtype)
+
+
 @pytest.mark.parametrize("rows", [1, 3, 9])
 @pytest.mark.parametrize("n", [40, 37, 1])
 def test_linear_of_operands_at_odd_addresses(rows, n):
