@@ -453,7 +453,7 @@ def test_gemv_rows(M, K1, K2, N):
 @pytest.mark.parametrize("M,N,K,rev", [(1, 4096, 4096, False), (8, 512, 4096, False), (32, 16384, 4096, True),
                                         (5, 4096, 16384, False), (64, 264, 520, True), (3, 50400, 1024, False)])
 def test_small_m_linear(M, N, K, rev):
-    """Decode-sized linear layers (split-K path) against fp32, and bit-identical when repeated."""
+    """Decode-sized linear layers (few-row products) against fp32, and bit-identical when repeated."""
     ops, co = _ops()
     torch.manual_seed(3)
     x = torch.randn(M, K, device="cuda", dtype=torch.bfloat16) * 0.5
